@@ -200,20 +200,30 @@ EncodeFn encode_fn() {
   return fn;
 }
 
+// A kernel's persistent grid on the current device: its shared-memory limit
+// set and its resident CTAs counted once per kernel and device.
 std::mutex g_attr_mu;
-std::unordered_map<uint64_t, bool> g_attr_done;
+std::unordered_map<uint64_t, int> g_resident;
 
-int ensure_smem(const void *func, size_t bytes) {
+int resident_ctas(const void *func, size_t bytes, int *ctas) {
   int dev = 0;
   cudaGetDevice(&dev);
   const uint64_t key = reinterpret_cast<uint64_t>(func) ^ ((uint64_t)dev << 56);
   std::lock_guard<std::mutex> lk(g_attr_mu);
-  if (g_attr_done.count(key)) return CCT_OK;
+  auto it = g_resident.find(key);
+  if (it != g_resident.end()) {
+    *ctas = it->second;
+    return CCT_OK;
+  }
   int rc = check_cuda(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)bytes),
                       "cudaFuncSetAttribute(direct_tma)");
-  if (!rc) g_attr_done[key] = true;
-  return rc;
+  if (rc) return rc;
+  int sms = 148, per_sm = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, kThreads, bytes);
+  *ctas = g_resident[key] = std::max(per_sm, 1) * sms;
+  return CCT_OK;
 }
 
 template <int R, int OFF>
@@ -227,16 +237,12 @@ int launch_tma(const ConvGeom &g, const float *x, const float *f, float *y, cuda
   const long long total = (long long)tiles_x * tiles_y * g.pout;
   if (total > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "direct convolution grid too large");
   auto kern = direct_tma_kernel<R, R, OFF>;
-  rc = ensure_smem((const void *)kern, T::SMEM);
-  if (rc) return rc;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // persistent CTAs: as many as are resident at once (registers and shared
   // memory decide), so no CTA waits for another to finish
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, T::SMEM);
-  const int grid = (int)std::min<long long>(total, (long long)std::max(per_sm, 1) * sms);
+  int resident = 0;
+  rc = resident_ctas((const void *)kern, T::SMEM, &resident);
+  if (rc) return rc;
+  const int grid = (int)std::min<long long>(total, resident);
   const int rc2 = launch_pdl(kern, dim3(grid), dim3(kThreads), T::SMEM, st, "direct_tma_kernel launch", map, g, f,
                              y, tiles_x, tiles_y, (int)total, err);
   if (!rc2) count_launches(1);
@@ -292,7 +298,12 @@ bool direct_tma_supported(const ConvGeom &g, const float *x) {
   if (g.R != g.S || (g.R != 1 && g.R != 3 && g.R != 5 && g.R != 7)) return false;
   if ((g.W & 3) != 0) return false;
   if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
-  return true;
+  // Fewer than 96 of these 64 x 128 tiles leave most SMs idle, and a field of
+  // at most 64 rows half of each tile: the direct stencils' smaller tiles are
+  // faster there (us, 5x5: one plane of 256x256 4.0 / 2.4, eight 4.2 / 3.7,
+  // sixteen 4.2 / 5.3; 512 planes of 60x64 9.1 / 7.4).
+  const long long tiles = (long long)((g.OW + kTW - 1) / kTW) * ((g.OH + kTH - 1) / kTH) * g.pout;
+  return tiles >= 96 && g.OH > 64;
 }
 
 int launch_direct_tma(const ConvGeom &g, const float *x, const float *f, float *y,
