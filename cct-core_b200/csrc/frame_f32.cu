@@ -4,13 +4,18 @@
 // (ConvolveHyperKernel.scala:153-199, 319-340, 574-645, fused by
 // ProjectFrameTensorReduceSumOptimizer.scala:75-170).
 //
-// One CTA owns a 32x16 output tile of one image for a block of 16 output
+// One CTA owns a 32x16 output tile of one image for a block of 4 or 16 output
 // planes.  It walks the N input planes in order; each plane's halo tile and
-// the 16 filters' taps for that plane are staged in shared memory with
-// cp.async, double-buffered so the next plane loads while this one computes.
-// A thread holds 4 adjacent outputs x 8 output planes.  Summation order per
-// output matches the reference (per-row fma chain, row sum, plane sum), so
+// the filters' taps for that plane are staged in shared memory with cp.async,
+// in three buffers, so the next two planes load while this one computes and
+// one barrier per plane suffices.
+// A thread holds 4 adjacent outputs x 4 or 8 output planes.  Summation order
+// per output matches the reference (per-row fma chain, row sum, plane sum), so
 // results are bit-identical to the FP32 CPU restatement.
+//
+// Bound: the FP32 pipe, R*S packed multiply-adds and R adds per output pair
+// (75 % busy on the B=16, C=32, K=64, 64x64, 5x5 layer: 0.165 ms, 41 TFLOP/s;
+// 0.269 ms with the staging's index arithmetic repeated for every plane).
 //
 // The same kernel without the reduce (REDUCE = false) serves the unfused
 // modes ProjectFrame / BackProjectFrame (CogFunctionAPI.scala:1370-1377,
@@ -25,31 +30,38 @@
 namespace cct {
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kU = 4;        // adjacent outputs per thread
-constexpr int kKT = 8;       // output planes per thread
-constexpr int kKG = 2;       // plane groups per CTA
-constexpr int kKB = kKT * kKG;  // output planes per CTA
 constexpr int kSX = 8, kSY = 16;  // spatial threads per group
 constexpr int kTW = kSX * kU, kTH = kSY;  // 32 x 16 output tile
 
-template <int R, int S, int DOWN>
+// KT output planes per thread, KG groups of threads: KT * KG output planes per
+// CTA.
+template <int R, int S, int DOWN, int KT, int KG>
 struct FrameTile {
+  static constexpr int KB = KT * KG, THREADS = kSX * kSY * KG;
   static constexpr int IN_COLS = (kTW - 1) * DOWN + S;
   static constexpr int IN_ROWS = (kTH - 1) * DOWN + R;
   static constexpr int PITCH = (IN_COLS + 3) & ~3;
   static constexpr int TILE = IN_ROWS * PITCH;
-  static constexpr int FILT = R * S * kKB;  // [tap][plane]
+  // [tap][plane], a tap every 4 or 20 floats: the taps a warp copies fall on 8
+  // different banks, and a tap's planes stay 16-byte aligned
+  static constexpr int FP = KB == 4 ? 4 : KB + 4;
+  static constexpr int FILT = R * S * FP;
   static constexpr int STAGE = TILE + FILT;
+  static constexpr int STAGES = 3;
+  static constexpr size_t SMEM = sizeof(float) * STAGES * STAGE;
+  // elements a thread copies per plane
+  static constexpr int NT = (IN_ROWS * IN_COLS + THREADS - 1) / THREADS, NF = (R * S * KB + THREADS - 1) / THREADS;
 };
 
-template <int R, int S, int DOWN, bool REDUCE>
-__global__ void __launch_bounds__(kThreads, 2)
+template <int R, int S, int DOWN, bool REDUCE, int KT, int KG>
+__global__ void __launch_bounds__(kSX * kSY * KG, KT == 8 ? 2 : 4)
     frame_f32_kernel(ConvGeom g, const float *__restrict__ x,
                      const float *__restrict__ f, float *__restrict__ y,
                      int tiles_x, int tiles_y, int kblocks, int tchunk) {
   grid_dependency_wait();  // launched with programmatic serialisation: nothing global before this
-  using T = FrameTile<R, S, DOWN>;
+  using T = FrameTile<R, S, DOWN, KT, KG>;
+  constexpr int kKT = KT, kKB = T::KB, kThreads = T::THREADS;
   constexpr int E = (kU - 1) * DOWN + S;
   constexpr int E4 = (E + 3) / 4;
   static_assert((kU * DOWN) % 4 == 0, "16-byte aligned thread origin");
@@ -70,8 +82,9 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int k0 = kb * kKB;
   const int kcount = min(kKB, g.groups - k0);
 
-  const int grp = threadIdx.x / (kSX * kSY);
-  const int sp = threadIdx.x % (kSX * kSY);
+  const int tid = threadIdx.x;
+  const int grp = tid / (kSX * kSY);
+  const int sp = tid % (kSX * kSY);
   const int tx = sp % kSX, ty = sp / kSX;
   const int out_r0 = ty_i * kTH, out_c0 = tx_i * kTW;
   const int org_r = out_r0 * DOWN - g.low_r;
@@ -79,23 +92,51 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int plane = g.H * g.W;
   const bool conv = g.orient == CCT_CONVOLUTION;
 
-  // Stage loader for input-plane term t into buffer `buf`.
-  auto issue = [&](int t, int buf) {
-    float *tile = smem + buf * T::STAGE;
+  // What a thread copies is the same for every input plane but for the plane's
+  // address, so the border mapping and the tap order are worked out once (done
+  // per plane, they were two fifths of the instructions).
+  int t_src[T::NT];  // offset in the input plane, -1 reads zero
+#pragma unroll
+  for (int e = 0; e < T::NT; ++e) {
+    const int i = tid + e * kThreads, tr = i / T::IN_COLS, tc = i - tr * T::IN_COLS;
+    const int sr = border_index(g.border, org_r + tr, g.H), sc = border_index(g.border, org_c + tc, g.W);
+    t_src[e] = (sr >= 0 && sc >= 0) ? sr * g.W + sc : -1;
+  }
+  // filter plane of (output plane k, input plane t): k*N + t, or t*K + k for
+  // the back-projected forms (plane_pair)
+  const bool back = g.mode == CCT_BACK_PROJECT_FRAME || g.mode == CCT_BACK_PROJECT_FRAME_BLOCK_REDUCE_SUM;
+  const size_t f_step = back ? (size_t)g.groups * (R * S) : (size_t)(R * S);
+  int f_src[T::NF];  // from the block's first filter plane
+#pragma unroll
+  for (int e = 0; e < T::NF; ++e) {
+    const int i = tid + e * kThreads, kk = i / (R * S), tap = i - kk * (R * S);
+    f_src[e] = min(kk, kcount - 1) * (back ? 1 : g.n) * (R * S) + (conv ? R * S - 1 - tap : tap);
+  }
+  const float *ft0 = f + (back ? (size_t)t0 * g.groups + k0 : (size_t)k0 * g.n + t0) * (R * S);
+  const float *xt = x + (size_t)(b * g.n + t0) * plane;
+  // Stage loader of input-plane term t (called in order).
+  auto issue = [&](int t) {
+    float *tile = smem + (t % T::STAGES) * T::STAGE;
     float *ft = tile + T::TILE;
-    const int ip = b * g.n + t0 + t;
-    load_tile_async(tile, T::PITCH, T::IN_ROWS, T::IN_COLS, x + (size_t)ip * plane, g, org_r, org_c);
-    for (int i = threadIdx.x; i < R * S * kKB; i += kThreads) {
-      const int kk = i / (R * S), tap = i - kk * (R * S);
-      const int r = tap / S, s = tap - r * S;
-      const int src_tap = conv ? (R - 1 - r) * S + (S - 1 - s) : tap;
-      // output plane of filter k0 + kk: b*K + k (reduced) or b*F + k*N + t
-      const int o = REDUCE ? b * g.groups + k0 + kk : b * g.pf + (k0 + kk) * g.n + t0 + t;
-      int ipp, fp;
-      plane_pair(g, o, REDUCE ? t : 0, &ipp, &fp);
-      const bool ok = kk < kcount;
-      cp_async_f32(ft + tap * kKB + kk, ok ? f + (size_t)fp * (R * S) + src_tap : f, ok);
+#pragma unroll
+    for (int e = 0; e < T::NT; ++e) {
+      const int i = tid + e * kThreads;
+      if (i < T::IN_ROWS * T::IN_COLS) {
+        const int tr = i / T::IN_COLS, tc = i - tr * T::IN_COLS;
+        cp_async_f32(tile + tr * T::PITCH + tc, t_src[e] >= 0 ? xt + t_src[e] : x, t_src[e] >= 0);
+      }
     }
+    const float *fp = ft0;
+    ft0 += f_step;
+#pragma unroll
+    for (int e = 0; e < T::NF; ++e) {
+      const int i = tid + e * kThreads;
+      if (i < R * S * kKB) {
+        const int kk = i / (R * S), tap = i - kk * (R * S);
+        cp_async_f32(ft + tap * T::FP + kk, fp + f_src[e], kk < kcount);
+      }
+    }
+    xt += plane;
     cp_async_commit();
   };
 
@@ -113,16 +154,19 @@ __global__ void __launch_bounds__(kThreads, 2)
   const bool relu = (g.flags & CCT_FLAG_RELU) != 0;
   const size_t opage = (size_t)g.OH * g.OW;
   const int row = out_r0 + ty;
-  issue(0, 0);
+  auto next = [&](int t) {  // an empty group past the last plane
+    if (t < nterms)
+      issue(t);
+    else
+      cp_async_commit();
+  };
+  next(0);
+  next(1);
   for (int t = 0; t < nterms; ++t) {
-    if (t + 1 < nterms) {
-      issue(t + 1, (t + 1) & 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const float *tile = smem + (t & 1) * T::STAGE;
+    cp_async_wait<1>();
+    __syncthreads();  // plane t has landed, and every thread is done with plane t - 1
+    next(t + 2);
+    const float *tile = smem + (t % T::STAGES) * T::STAGE;
     const float *ft = tile + T::TILE + grp * kKT;
     const float *base = tile + (ty * DOWN) * T::PITCH + tx * kU * DOWN;
 
@@ -149,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         float2 w[kP];
 #pragma unroll
         for (int k4 = 0; k4 < kKT / 4; ++k4) {
-          const float4 q = *reinterpret_cast<const float4 *>(ft + (r * S + s) * kKB + 4 * k4);
+          const float4 q = *reinterpret_cast<const float4 *>(ft + (r * S + s) * T::FP + 4 * k4);
           w[2 * k4 + 0] = make_float2(q.x, q.y);
           w[2 * k4 + 1] = make_float2(q.z, q.w);
         }
@@ -196,7 +240,6 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
       }
     }
-    __syncthreads();
   }
 
   if constexpr (REDUCE) {
@@ -216,23 +259,45 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
-template <int R, int S, int DOWN>
-int launch(const ConvGeom &g, const float *x, const float *f, float *y, cudaStream_t st) {
-  const bool reduce = g.mode == CCT_PROJECT_FRAME_BLOCK_REDUCE_SUM || g.mode == CCT_BACK_PROJECT_FRAME_BLOCK_REDUCE_SUM;
-  using T = FrameTile<R, S, DOWN>;
+template <int R, int S, int DOWN, bool REDUCE, int KT, int KG>
+int launch_k(const ConvGeom &g, const float *x, const float *f, float *y, cudaStream_t st) {
+  using T = FrameTile<R, S, DOWN, KT, KG>;
   const int tiles_x = (g.OW + kTW - 1) / kTW, tiles_y = (g.OH + kTH - 1) / kTH;
-  const int kblocks = (g.groups + kKB - 1) / kKB;
-  const int tchunk = reduce ? g.terms : 4;  // unfused: 4 input planes per CTA
-  const int nchunks = reduce ? 1 : (g.n + tchunk - 1) / tchunk;
+  const int kblocks = (g.groups + T::KB - 1) / T::KB;
+  const int tchunk = REDUCE ? g.terms : 4;  // unfused: 4 input planes per CTA
+  const int nchunks = REDUCE ? 1 : (g.n + tchunk - 1) / tchunk;
   const long long blocks = (long long)tiles_x * tiles_y * kblocks * nchunks * g.batch;
   if (blocks > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "frame grid too large");
-  const size_t smem = 2 * sizeof(float) * T::STAGE;
-  static_assert(2 * sizeof(float) * T::STAGE <= 48 * 1024, "frame stages exceed the default smem limit");
-  const int rc = launch_pdl(reduce ? frame_f32_kernel<R, S, DOWN, true> : frame_f32_kernel<R, S, DOWN, false>,
-                            dim3((unsigned)blocks), dim3(kThreads), smem, st, "frame_f32_kernel launch", g, x, f, y,
-                            tiles_x, tiles_y, kblocks, tchunk);
+  const auto kern = frame_f32_kernel<R, S, DOWN, REDUCE, KT, KG>;
+  if (T::SMEM > 48 * 1024) {
+    const int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM),
+                              "cudaFuncSetAttribute(frame_f32)");
+    if (rc) return rc;
+  }
+  const int rc = launch_pdl(kern, dim3((unsigned)blocks), dim3(T::THREADS), T::SMEM, st,
+                            "frame_f32_kernel launch", g, x, f, y, tiles_x, tiles_y, kblocks, tchunk);
   if (!rc) count_launches(1);
   return rc;
+}
+
+template <int R, int S, int DOWN>
+int launch(const ConvGeom &g, const float *x, const float *f, float *y, cudaStream_t st) {
+  if (g.mode != CCT_PROJECT_FRAME_BLOCK_REDUCE_SUM && g.mode != CCT_BACK_PROJECT_FRAME_BLOCK_REDUCE_SUM)
+    return launch_k<R, S, DOWN, false, 8, 2>(g, x, f, y, st);
+  // 16 output planes per CTA re-use a staged tile four times as often, which
+  // pays for filters of up to 3x3 while that grid fills the SMs; larger filters
+  // are bound by the multiply-adds either way, and four times the CTAs spread
+  // better (us, 16 / 4 planes per CTA: 3x3 32 -> 64 planes on 16x 64x64, 512 CTAs
+  // 83 / 93; 3x3 32 -> 16 on 64x 32x32, 128 CTAs 26 / 30; 3x3 64 -> 64 on 8x 32x32,
+  // 64 CTAs 48 / 32; 5x5 32 -> 64 on 16x 64x64 169 / 165; 7x7 309 / 285; 5x5
+  // 32 -> 32 on 4x 48x48 49 / 29).
+  const long long blocks16 = (long long)((g.OW + kTW - 1) / kTW) * ((g.OH + kTH - 1) / kTH) * g.batch *
+                             ((g.groups + 15) / 16);
+  const bool full16 = (g.groups + 15) / 16 * 16 * 4 <= g.groups * 5;  // at most a fifth of the planes idle
+  if constexpr (R <= 3) {
+    if (blocks16 >= 128 && full16) return launch_k<R, S, DOWN, true, 8, 2>(g, x, f, y, st);
+  }
+  return launch_k<R, S, DOWN, true, 4, 1>(g, x, f, y, st);
 }
 
 }  // namespace
@@ -243,6 +308,8 @@ bool frame_f32_supported(const ConvGeom &g) {
     return false;
   if (g.up != 1) return false;
   if (g.R != g.S) return false;
+  // a block's filter offsets and a plane's element offsets are 32-bit
+  if (16LL * g.n * g.R * g.S > 0x7fffffffLL || (long long)g.H * g.W > 0x7fffffffLL) return false;
   if (g.down != 1 && g.down != 2) return false;
   return g.R == 1 || g.R == 3 || g.R == 5 || g.R == 7 || g.R == 9;
 }
