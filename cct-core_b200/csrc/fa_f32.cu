@@ -13,8 +13,10 @@
 // j from 0 per gradient row, row sums added in order, so the result is
 // bit-identical to the FP32 oracle.
 //
-// fa_rows_kernel (the main path): a CTA serves one image b, kCG input planes
-// and kLG gradient planes.  It streams the gradient rows i = 0.. through
+// fa_quad_kernel: the main path, described below.
+// fa_rows_kernel (fields too wide for its shared memory): a CTA serves one
+// image b, kCG input planes and kLG gradient planes.  It streams the gradient
+// rows i = 0.. through
 // shared memory together with a ring of the OH image rows each step needs
 // (cp.async, the next rows landing while the current ones are used), so
 // every image row and gradient row is read from L2 once per CTA.
@@ -24,6 +26,7 @@
 // The block-reduced form writes the per-image results to plan workspace and
 // a second kernel adds them in image order.
 #include "cct_internal.h"
+#include "sm100_util.cuh"
 #include "tile_common.cuh"
 
 namespace cct {
@@ -130,6 +133,190 @@ __global__ void __launch_bounds__(kCG * kLG * kFaMaxS)
   for (int s = 0; s < S; ++s) yp[s] = relu ? fmaxf(acc[s], 0.0f) : acc[s];
 }
 
+// fa_quad_kernel (the main path): a lane owns one (input plane, result row)
+// and four gradient planes, so an image value feeds 4 S multiply-adds and a
+// float4 of the four planes' gradients comes as one broadcast read; a warp
+// owns a gradient row i of the step, kQRows warps the step's rows.  Row sums
+// meet in shared memory and are added in row order by the thread that keeps
+// the output, so splitting the rows over warps does not change the order.
+// Gradient planes l, l+1 advance together in packed fma.rn.f32x2 (each lane
+// the scalar RN operation).
+//
+// Bound: the FP32 pipe (2 S packed multiply-adds per gradient column; half busy,
+// the 16 warps that shared memory leaves an SM wait on their chains): 0.22 ms for
+// the weight gradient of the B=16, C=32, K=64, 64x64, 5x5 layer.  fa_rows_kernel
+// read an image and a gradient value from shared memory per S multiply-adds: L1
+// 91 % busy, 0.62 ms.
+// NW gradient rows per step, one per warp: 4, or 8 or 16 where the grid leaves
+// SMs idle and the steps' latency is what the launch waits for.
+constexpr int kQL = 4;                   // gradient planes per CTA
+constexpr size_t kQuadSmemMax = 220 * 1024;
+
+// input planes a warp's 32 consecutive (plane, row) pairs can touch
+__host__ __device__ inline int quad_planes(const ConvGeom &g) {
+  const int n = (32 + g.OH - 2) / g.OH + 1;
+  return n < g.n ? n : g.n;
+}
+__host__ __device__ inline int quad_ring(int OH, int NW) { return 2 * NW + OH - 1; }
+// row pitch: whole float4s past the last window, an odd number of them so that
+// neighbouring ring rows start on different banks
+__host__ __device__ inline int quad_pitch(const ConvGeom &g) {
+  const int n4 = (g.S + 3) / 4 + (g.OW + 6) / 4;
+  return 4 * (n4 | 1);
+}
+inline size_t quad_smem(const ConvGeom &g, int NW) {
+  return sizeof(float) * ((size_t)quad_planes(g) * quad_ring(g.OH, NW) * quad_pitch(g) +
+                          2 * (size_t)NW * kQL * ((g.S + 3) & ~3) + (size_t)NW * kQL * g.OW * 32);
+}
+
+template <int S, int NW>
+__global__ void __launch_bounds__(NW * 32)
+    fa_quad_kernel(ConvGeom g, const float *__restrict__ x, const float *__restrict__ f, float *__restrict__ y,
+                   int mgroups, int lgroups) {
+  extern __shared__ __align__(16) float sm[];
+  grid_dependency_wait();  // launched with programmatic serialisation: nothing global before this
+  constexpr int NT = NW * 32, NV = (S + 6) / 4, OUTS = kQL * S * 32, NO = (OUTS + NT - 1) / NT;
+  const int Hg = g.R, Wg = g.S, C = g.n, L = g.groups, B = g.batch, OH = g.OH, W = g.W;
+  const int pitch = quad_pitch(g), ring = quad_ring(OH, NW), gcols = (Wg + 3) & ~3;
+  float *xr = sm;                                                       // [plane][ring][pitch]
+  float *gr = xr + (size_t)quad_planes(g) * ring * pitch;              // [2][row][column][plane]
+  float *sums = gr + 2 * NW * kQL * gcols;                          // [row][(plane, s)][lane]
+  int bid = blockIdx.x;
+  const int m0 = (bid % mgroups) * 32;
+  bid /= mgroups;
+  const int l0 = (bid % lgroups) * kQL, b = bid / lgroups;
+  const int c0 = m0 / OH, nc = min(C, (m0 + 31) / OH + 1) - c0, nl = min(kQL, L - l0);
+  const bool conv = g.orient == CCT_CONVOLUTION;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = min(m0 + lane, C * OH - 1), cl = m / OH - c0, r = m - (m / OH) * OH;
+  const bool wide = (W & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+
+  // One image row of every plane of the group into its ring slot (a warp).
+  const float *xg = x + (size_t)(b * C + c0) * g.H * W;
+  const int cstride = ring * pitch, lane4 = 4 * lane;
+  auto load_x = [&](int row, int slot) {
+    const float *src = xg + (size_t)row * W + (wide ? lane4 : lane);
+    float *dst = xr + slot * pitch + (wide ? lane4 : lane);
+    const size_t page = (size_t)g.H * W;
+    for (int c = 0; c < nc; ++c, src += page, dst += cstride) {
+      if (wide) {
+        for (int col = 0; col + lane4 < W; col += 128) cp_async_16(dst + col, src + col, true);
+      } else {
+        for (int col = 0; col + lane < W; col += 32) cp_async_f32(dst + col, src + col, true);
+      }
+    }
+  };
+  // This warp's gradient row i (flipped for convolution) of the four planes,
+  // a column's planes adjacent.
+  const float *fg = f + (size_t)(b * L + l0) * Hg * Wg;
+  const size_t gpage = (size_t)Hg * Wg;
+  const int jstep = conv ? -32 : 32;
+  auto load_g = [&](int i, float *buf) {
+    const float *src = fg + (size_t)(conv ? Hg - 1 - i : i) * Wg + (conv ? Wg - 1 - lane : lane);
+    float *dst = buf + (size_t)warp * gcols * kQL + lane * kQL;
+    for (int j = lane; j < Wg; j += 32, src += jstep, dst += 32 * kQL)
+#pragma unroll
+      for (int l = 0; l < kQL; ++l) cp_async_f32(dst + l, l < nl ? src + l * gpage : f, l < nl);
+  };
+
+  const int steps = (Hg + NW - 1) / NW;
+  for (int row = warp; row < min(NW, Hg) + OH - 1; row += NW) load_x(row, row);
+  if (warp < Hg) load_g(warp, gr);
+  cp_async_commit();
+
+  // ring slots of the row this lane reads at step k (i0 + warp + r) and of the
+  // row this warp loads for the next step (i0 + NW + OH - 1 + warp)
+  int rslot = (warp + r) % ring, lslot = (NW + OH - 1 + warp) % ring;
+  float acc[NO];
+#pragma unroll
+  for (int o = 0; o < NO; ++o) acc[o] = 0.0f;
+  for (int k = 0; k < steps; ++k) {
+    const int i0 = k * NW, rows = min(NW, Hg - i0);
+    cp_async_wait<0>();
+    __syncthreads();  // this step's rows have landed; the last step's sums are added
+    if (i0 + NW + warp < Hg) {
+      load_x(i0 + NW + OH - 1 + warp, lslot);
+      load_g(i0 + NW + warp, gr + ((k + 1) & 1) * NW * kQL * gcols);
+    }
+    cp_async_commit();
+    if (warp < rows) {
+      const float4 *xp = reinterpret_cast<const float4 *>(xr + (size_t)cl * cstride + rslot * pitch);
+      const float4 *gp = reinterpret_cast<const float4 *>(gr + ((k & 1) * NW + warp) * kQL * gcols);
+      float2 cs[S][2];
+#pragma unroll
+      for (int s = 0; s < S; ++s) cs[s][0] = cs[s][1] = make_float2(0.0f, 0.0f);
+      // the image values of columns 4 q .. 4 (q + NV) - 1, each twice (the
+      // packed form's operand), float4 number n at place n mod NV: NV quads of
+      // columns are unrolled, so that the window never moves
+      float2 win[4 * NV];
+      auto put = [&](int e, const float4 v) {
+        win[4 * e + 0] = make_float2(v.x, v.x);
+        win[4 * e + 1] = make_float2(v.y, v.y);
+        win[4 * e + 2] = make_float2(v.z, v.z);
+        win[4 * e + 3] = make_float2(v.w, v.w);
+      };
+      auto tap = [&](int first, const float4 v) {  // one gradient column
+        const float2 g0 = make_float2(v.x, v.y), g1 = make_float2(v.z, v.w);
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          const float2 xv = win[(first + s) % (4 * NV)];
+          cs[s][0] = __ffma2_rn(xv, g0, cs[s][0]);
+          cs[s][1] = __ffma2_rn(xv, g1, cs[s][1]);
+        }
+      };
+#pragma unroll
+      for (int e = 0; e < NV; ++e) put(e, xp[e]);
+      const int quads = Wg / 4, rest = Wg - 4 * quads;
+      for (int q = 0; q <= quads; q += NV) {
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+          if (q + u < quads) {
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) tap(4 * u + jj, gp[4 * (q + u) + jj]);
+            put(u, xp[q + u + NV]);
+          } else if (q + u == quads) {
+#pragma unroll
+            for (int jj = 0; jj < 3; ++jj)
+              if (jj < rest) tap(4 * u + jj, gp[4 * quads + jj]);
+          }
+        }
+      }
+      float *out = sums + (size_t)warp * OUTS + lane;
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        out[(0 * S + s) * 32] = cs[s][0].x;
+        out[(1 * S + s) * 32] = cs[s][0].y;
+        out[(2 * S + s) * 32] = cs[s][1].x;
+        out[(3 * S + s) * 32] = cs[s][1].y;
+      }
+    }
+    rslot += NW;
+    if (rslot >= ring) rslot -= ring;
+    lslot += NW;
+    if (lslot >= ring) lslot -= ring;
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < NO; ++o) {
+      const int q = o * NT + threadIdx.x;
+      if (OUTS % NT == 0 || q < OUTS) {
+#pragma unroll 4
+        for (int i = 0; i < rows; ++i) acc[o] = __fadd_rn(acc[o], sums[i * OUTS + q]);
+      }
+    }
+  }
+  allow_dependent_launch();
+  const bool relu = (g.flags & CCT_FLAG_RELU) != 0;
+#pragma unroll
+  for (int o = 0; o < NO; ++o) {
+    const int q = o * NT + threadIdx.x, l = q / (32 * S), s = (q >> 5) - l * S, mm = m0 + (q & 31);
+    if ((OUTS % NT == 0 || q < OUTS) && l < nl && mm < C * OH) {
+      const int c = mm / OH, rr = mm - c * OH;
+      float *yp = y + ((size_t)B * ((size_t)(l0 + l) * C + c) + b) * OH * S + (size_t)rr * S;
+      yp[s] = relu ? fmaxf(acc[o], 0.0f) : acc[o];
+    }
+  }
+}
+
 template <int S>
 __global__ void __launch_bounds__(kFaThreads)
     fa_f32_kernel(ConvGeom g, const float *__restrict__ x, const float *__restrict__ f, float *__restrict__ y,
@@ -223,7 +410,36 @@ int launch_fa_f32(const ConvGeom &g, const float *x, const float *f, float *y, f
   ConvGeom q = g;
   if (reduce) q.flags &= ~CCT_FLAG_RELU;  // ReLU applies to the reduced sum
   const size_t rsmem = fa_rows_smem(g);
-  if (g.OH <= kFaMaxS && rsmem <= kRowsSmemMax) {
+  const long long mgroups = ((long long)g.n * g.OH + 31) / 32, qlgroups = (g.groups + kQL - 1) / kQL;
+  const long long qblocks = g.batch * qlgroups * mgroups;
+  // up to 400 CTAs: as many rows per step as shared memory holds (us with 16 /
+  // 4: 96 CTAs of a 3x3 64 -> 64 layer on 64x64 26 / 63, 160 of a 5x5 32 -> 32
+  // on 4x 48x48 39 / 47, 384 of a 3x3 64 -> 64 on 4x 32x32 28 / 32; 1280 of a
+  // 5x5 32 -> 64 on 16x 64x64 248 / 224)
+  const int nw = qblocks > 400 ? 4 : quad_smem(g, 16) <= kQuadSmemMax ? 16 : quad_smem(g, 8) <= kQuadSmemMax ? 8 : 4;
+  const size_t qsmem = quad_smem(g, nw);
+  if (g.OH <= kFaMaxS && qsmem <= kQuadSmemMax && qblocks <= 0x7fffffffLL && (long long)g.n * g.OH < (1 << 30)) {
+#define CCT_FA_QUAD_CASE(SS)                                                                                  \
+  case SS: {                                                                                                  \
+    const auto kern = nw == 16 ? fa_quad_kernel<SS, 16> : nw == 8 ? fa_quad_kernel<SS, 8> : fa_quad_kernel<SS, 4>; \
+    if (qsmem > 48 * 1024) {                                                                                  \
+      int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsmem), \
+                          "cudaFuncSetAttribute(fa quad)");                                                   \
+      if (rc) return rc;                                                                                      \
+    }                                                                                                         \
+    int rc = launch_pdl(kern, dim3((unsigned)qblocks), dim3(nw * 32), qsmem, st,                              \
+                        "fa_quad_kernel launch", q, x, f, dst, (int)mgroups, (int)qlgroups);                  \
+    if (rc) return rc;                                                                                        \
+    break;                                                                                                    \
+  }
+    switch (g.OW) {
+      CCT_FA_QUAD_CASE(1) CCT_FA_QUAD_CASE(2) CCT_FA_QUAD_CASE(3) CCT_FA_QUAD_CASE(4)
+      CCT_FA_QUAD_CASE(5) CCT_FA_QUAD_CASE(6) CCT_FA_QUAD_CASE(7) CCT_FA_QUAD_CASE(8)
+      default: return set_error(CCT_ENOTSUP, "FilterAdjoint result width %d", g.OW);
+    }
+#undef CCT_FA_QUAD_CASE
+    count_launches(1);
+  } else if (g.OH <= kFaMaxS && rsmem <= kRowsSmemMax) {
     const int cgroups = (g.n + kCG - 1) / kCG, lgroups = (g.groups + kLG - 1) / kLG;
     const long long rblocks = (long long)g.batch * lgroups * cgroups;
     if (rblocks > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "FilterAdjoint grid too large");

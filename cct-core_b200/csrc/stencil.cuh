@@ -13,13 +13,6 @@ __device__ __forceinline__ int stencil_index(int border, int v, int n) {
   return border_index(border, v, n);
 }
 
-// cp.async of 16 bytes (both addresses 16-byte aligned), or 16 zero bytes.
-__device__ __forceinline__ void cp_async_16(float *dst, const float *src, bool valid) {
-  const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 16 : 0)
-               : "memory");
-}
-
 // Copies rows x COLS border-mapped values whose corner is (org_r, org_c) into
 // tile[row * PITCH + col].  A thread owns fixed columns of every row it copies,
 // so a column is mapped by the border once per tile and an element costs an

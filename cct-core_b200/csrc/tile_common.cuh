@@ -78,6 +78,12 @@ __device__ __forceinline__ void cp_async_f32(float *dst, const float *src,
                "l"(src), "r"(valid ? 4 : 0)
                : "memory");
 }
+// cp.async of 16 bytes (both addresses 16-byte aligned), or 16 zero bytes.
+__device__ __forceinline__ void cp_async_16(float *dst, const float *src, bool valid) {
+  const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
