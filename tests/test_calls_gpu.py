@@ -83,3 +83,26 @@ def test_color_calls(border):
         od = O.make_desc(rows, cols, R, R, border=_BORDERS[border])
         got = C.convolve(torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda(), border)
         assert np.array_equal(got.cpu().numpy(), O.color_conv(od, x, f))
+
+
+# tall and short tiles, a last tile of one row or column, 16- and 4-byte stores,
+# fields smaller than the filter
+@pytest.mark.parametrize("border", [O.ZERO, O.CLAMP, O.CYCLIC, O.VALID, O.FULL])
+@pytest.mark.parametrize("R", [1, 3, 5, 7])
+@pytest.mark.parametrize("rows,cols", [(33, 65), (8, 64), (9, 7), (330, 961), (321, 960)])
+def test_color_stencil(rows, cols, R, border):
+    rng = np.random.default_rng(rows * cols + R)
+    x = rng.integers(0, 256, (rows, cols, 4), dtype=np.uint8)
+    f = rng.uniform(-0.1, 1.0 / R, (R, R)).astype(np.float32)
+    od = O.make_desc(rows, cols, R, R, border=border, orient=O.XCORR)
+    d = _lib.new_desc(image_rows=rows, image_cols=cols, filter_rows=R, filter_cols=R, border=border,
+                      orientation=_lib.CROSS_CORRELATION, algo=_lib.ALGO_DIRECT)
+    plan = _lib.ColorPlan(d)
+    xd, fd = torch.from_numpy(x).cuda(), torch.from_numpy(f).cuda()
+    for static in (False, True):
+        if static:
+            plan.set_static_filter(f.ctypes.data)
+        y = torch.zeros((plan.shape[0], plan.shape[1], 4), device="cuda", dtype=torch.uint8)
+        plan.run(xd.data_ptr(), 0 if static else fd.data_ptr(), y.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert np.array_equal(y.cpu().numpy(), O.color_conv(od, x, f))
+    plan.close()
