@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kSmThreads, R == 7 ? 3 : 4)
 }
 
 // ---------------------------------------------------------------------------
-// Wide filters: S odd, 9..31, any R, no sampling, one term.  Weights come from
+// Wide filters: S odd, 3..63, any R, no sampling, one term.  Weights come from
 // shared memory as broadcast float4s, so a thread owns 8 adjacent columns: a
 // weight load feeds 32 multiply-adds and the row of 8 + S - 1 inputs it holds
 // in registers feeds V output rows (one input per multiply-add came from
@@ -644,7 +644,10 @@ int launch_direct(const ConvGeom &g, const float *x, const float *f, float *y,
     switch (g.S) {
       CCT_WIDE_CASE(3) CCT_WIDE_CASE(5) CCT_WIDE_CASE(7) CCT_WIDE_CASE(9) CCT_WIDE_CASE(11) CCT_WIDE_CASE(13)
       CCT_WIDE_CASE(15) CCT_WIDE_CASE(17) CCT_WIDE_CASE(19) CCT_WIDE_CASE(21) CCT_WIDE_CASE(23) CCT_WIDE_CASE(25)
-      CCT_WIDE_CASE(27) CCT_WIDE_CASE(29) CCT_WIDE_CASE(31)
+      CCT_WIDE_CASE(27) CCT_WIDE_CASE(29) CCT_WIDE_CASE(31) CCT_WIDE_CASE(33) CCT_WIDE_CASE(35) CCT_WIDE_CASE(37)
+      CCT_WIDE_CASE(39) CCT_WIDE_CASE(41) CCT_WIDE_CASE(43) CCT_WIDE_CASE(45) CCT_WIDE_CASE(47) CCT_WIDE_CASE(49)
+      CCT_WIDE_CASE(51) CCT_WIDE_CASE(53) CCT_WIDE_CASE(55) CCT_WIDE_CASE(57) CCT_WIDE_CASE(59) CCT_WIDE_CASE(61)
+      CCT_WIDE_CASE(63)
       default: break;
     }
 #undef CCT_WIDE_CASE

@@ -116,3 +116,11 @@ def test_up_bank(mode, rows, cols, R, step):
     ref = O.conv(od, x, f)
     assert bitwise_equal(_run(od, x, f), ref)
     assert bitwise_equal(_run(od, x, f, flags=_lib.FLAG_RELU), np.maximum(ref, 0))
+
+
+# the widths past 31, which take the short tile only
+@pytest.mark.parametrize("S", list(range(33, 65, 2)))
+@pytest.mark.parametrize("rows,cols,planes,R,border", [(17, 66, 2, 33, "clamp"), (40, 70, 1, 63, "cyclic"),
+                                                       (16, 64, 0, 1, "zero")])
+def test_widest(S, rows, cols, planes, R, border):
+    _check(rows, cols, R, S, border, O.CONV if S % 4 == 1 else O.XCORR, planes=planes)
