@@ -220,6 +220,7 @@ struct cct_conv_plan {
   FftParams fft;         // FFT plan (ALGO_FFT)
   float2 *fft_spec;      // working spectrum (plan workspace)
   float2 *fft_filter;    // filter spectrum
+  float2 *fft_rows;      // row transforms of a dynamic filter
   float2 *fft_tw;        // twiddle tables
   bool fft_static;       // fft_filter holds the static filter's FP64 spectrum
   float *fa_work;        // per-image FilterAdjoint results before the block reduce
@@ -463,6 +464,7 @@ int cct_conv_plan_create(const cct_conv_desc *d, cct_conv_plan **out) {
     if (!rc)
       rc = check_cuda(cudaMalloc(&p->fft_filter, fp.filter_elems * sizeof(float2)),
                       "cudaMalloc(fft filter spectrum)");
+    if (!rc) rc = check_cuda(cudaMalloc(&p->fft_rows, fp.row_elems * sizeof(float2)), "cudaMalloc(fft filter rows)");
     if (!rc) rc = check_cuda(cudaMalloc(&p->fft_tw, fp.tw_elems * sizeof(float2)), "cudaMalloc(fft twiddles)");
     if (!rc) {
       std::vector<float> tw;
@@ -486,6 +488,7 @@ int cct_conv_plan_destroy(cct_conv_plan *p) {
   cudaFree(p->packed);
   cudaFree(p->fft_spec);
   cudaFree(p->fft_filter);
+  cudaFree(p->fft_rows);
   cudaFree(p->fft_tw);
   cudaFree(p->fa_work);
   cudaFree(p->d_x);
@@ -550,11 +553,8 @@ int cct_conv_run(const cct_conv_plan *p, const float *x, const float *f, float *
     case ALGO_FILTER_ADJOINT_BF16X3:
       return launch_fa_tc(p->g, x, f, y, p->fa_work, p->err, st);
     case ALGO_FFT: {
-      int rc = CCT_OK;
-      if (f != p->static_filter || !p->fft_static)
-        rc = launch_fft_filter_spectrum(p->fft, f, p->fft_filter, st);
-      if (rc) return rc;
-      return launch_fft_conv(p->fft, x, p->fft_filter, p->fft_spec, y, st);
+      const bool dynamic = f != p->static_filter || !p->fft_static;
+      return launch_fft_conv(p->fft, x, dynamic ? f : nullptr, p->fft_rows, p->fft_filter, p->fft_spec, y, st);
     }
     default:
       if (direct_tma_supported(p->g, x)) return launch_direct_tma(p->g, x, f, y, st, p->err);

@@ -13,18 +13,24 @@
 // Three kernels per run:
 //   fft_rows_r2c   expanded rows (Fc reals packed as N = Fc/2 complex): N-point
 //                  FFT, then the even/odd split to the Fc/2 + 1 non-negative
-//                  frequencies;
+//                  frequencies.  Only the grid rows that hold the field and the
+//                  border its outputs can read are transformed (the others are
+//                  zero or are never read); the R rows of a dynamic filter go
+//                  along in the same launch;
 //   fft_cols       blocks of spectrum columns: Fr-point FFT down each
-//                  column, times G, inverse FFT (or, for a dynamic filter's
-//                  spectrum, forward FFT and scaling only);
+//                  column, times G, inverse FFT (before it, for a dynamic
+//                  filter, a launch that makes G: forward FFT and scaling only);
 //   fft_rows_c2r   output rows: inverse of the split, N-point inverse FFT,
 //                  unpacked and trimmed to the field.
 // Each FFT is a Stockham autosort in radix-16 passes (radix 2/4/8 for the
 // last): every thread keeps 16 complex values in registers and does one
 // 16-point (or 16/R R-point) DFT per pass, so an N-point FFT takes
-// ceil(log2 N / 4) shared-memory exchanges.  Shared-memory sequences are
-// padded by one element every 16 so the strided exchanges stay free of bank
-// conflicts.  Twiddles are computed in FP64 on the host and stored as float2.
+// ceil(log2 N / 4) passes and one shared-memory exchange fewer: the last pass
+// leaves thread tt the elements tt + m T, which are what the first pass of the
+// inverse takes and what a column or an output row stores.  Shared-memory
+// sequences are padded by one element every 16 so the strided exchanges stay
+// free of bank conflicts.  Twiddles are computed in FP64 on the host and stored
+// as float2.
 #include <cmath>
 #include <complex>
 #include <vector>
@@ -37,9 +43,17 @@
 namespace cct {
 namespace {
 
-constexpr int kRowThreads = 256;
-constexpr int kColThreads = 512;
-__host__ __device__ constexpr int col_stride(int Fr) { return Fr + Fr / 16 + 8; }
+// Threads of a row CTA (as many rows as they hold) and of a column CTA: four
+// columns, or more while that leaves fewer than 64 threads.
+__host__ __device__ constexpr int row_threads(int N) { return N / 16 > 64 ? N / 16 : 64; }
+__host__ __device__ constexpr int col_width(int Fr) { return Fr / 16 * 4 >= 64 ? 4 : 64 / (Fr / 16); }
+// Shared-memory stride of a column in complex values: a warp holds 32/CW
+// consecutive elements of each of CW columns, so a stride of 32/CW (mod 16)
+// spreads its 32 values evenly over the banks.
+__host__ __device__ constexpr int col_stride(int Fr) {
+  const int base = Fr + Fr / 16, cw = col_width(Fr), want = cw >= 32 ? 1 : 32 / cw;
+  return base + ((want - base) % 16 + 16) % 16;
+}
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -194,21 +208,32 @@ __device__ __forceinline__ void pass_store(float2 *s, const float2 (&v)[16], int
   }
 }
 
-// N-point FFT (N = 2^LOGN >= 16) of the sequence whose first-pass inputs
-// v[m] = x[tt + m*T] the caller loaded; the result lands in natural order in
-// s (padded).  The passes (radix 16, the last 2..16) are fixed at compile
-// time.  Every thread of the CTA takes part (the passes synchronise the CTA).
-template <int LOGN, bool INV, int NS_LOG = 0, bool FIRST = true>
-__device__ __forceinline__ void fft_passes(float2 *s, float2 (&v)[16], int tt, const float2 *__restrict__ tw) {
-  if constexpr (NS_LOG < LOGN) {
-    constexpr int B = (LOGN - NS_LOG) >= 4 ? 4 : (LOGN - NS_LOG);
-    constexpr int R = 1 << B, N = 1 << LOGN, T = N / 16;
-    if (!FIRST) pass_load<R>(s, v, N, T, tt);
-    pass_compute<R, INV>(v, N, 1 << NS_LOG, T, tt, tw);
-    __syncthreads();
+// N-point FFT (N = 2^LOGN >= 16) of the sequence whose elements tt + m T the
+// caller holds in v[m]; leaves thread tt the elements tt + m T of the result in
+// v[m] (the last pass, of radix R, computes X[tt + T (q + m 16/R)] in v[q R + m]).
+// The passes (radix 16, the last 2..16) are fixed at compile time.  Every
+// thread of the CTA takes part (the passes synchronise the CTA); SYNC: others
+// may still read s when this starts.
+template <int LOGN, bool INV, bool SYNC, int NS_LOG = 0>
+__device__ __forceinline__ void fft_regs(float2 *s, float2 (&v)[16], int tt, const float2 *__restrict__ tw) {
+  constexpr int B = (LOGN - NS_LOG) >= 4 ? 4 : (LOGN - NS_LOG);
+  constexpr int R = 1 << B, N = 1 << LOGN, T = N / 16;
+  pass_compute<R, INV>(v, N, 1 << NS_LOG, T, tt, tw);
+  if constexpr (NS_LOG + B < LOGN) {
+    constexpr int R2 = 1 << ((LOGN - NS_LOG - B) >= 4 ? 4 : (LOGN - NS_LOG - B));
+    if (SYNC || NS_LOG > 0) __syncthreads();
     pass_store<R>(s, v, 1 << NS_LOG, T, tt);
     __syncthreads();
-    fft_passes<LOGN, INV, NS_LOG + B, false>(s, v, tt, tw);
+    pass_load<R2>(s, v, N, T, tt);
+    fft_regs<LOGN, INV, SYNC, NS_LOG + B>(s, v, tt, tw);
+  } else if constexpr (R < 16) {
+    float2 t[16];
+#pragma unroll
+    for (int q = 0; q < 16 / R; ++q)
+#pragma unroll
+      for (int m = 0; m < R; ++m) t[q + m * (16 / R)] = v[q * R + m];
+#pragma unroll
+    for (int m = 0; m < 16; ++m) v[m] = t[m];
   }
 }
 
@@ -233,28 +258,35 @@ __device__ __forceinline__ int filter_index(int pos, int h, int R, int F, bool c
   return (r >= 0 && r < R) ? r : -1;
 }
 
-// Row pass: rows_per_cta sequences of N = Fc/2 complex points per CTA.
-// SRC 0: image plane rows expanded with the border; 1: filter plane rows
-// centred at the origin (flipped for convolution).
-template <int SRC, int LOGN>
-__global__ void __launch_bounds__(kRowThreads, 4)
-    fft_rows_r2c(FftParams p, const float *__restrict__ src, float2 *__restrict__ spec, int planes) {
+// Row pass: row_threads/T sequences of N = Fc/2 complex points per CTA.  The
+// first planes * (top + bottom) sequences are the image planes' grid rows,
+// expanded with the border, into spec; the rest the rows of the filter planes
+// (centred at the origin, flipped for convolution), into rows.
+template <int LOGN>
+__global__ void __launch_bounds__(row_threads(1 << LOGN), 1024 / row_threads(1 << LOGN))
+    fft_rows_r2c(FftParams p, const float *__restrict__ x, const float *__restrict__ f, float2 *__restrict__ spec,
+                 float2 *__restrict__ rows, int planes, int fplanes) {
   extern __shared__ __align__(16) float2 fsm[];
   grid_dependency_wait();  // launched with programmatic serialisation
   allow_dependent_launch();
-  constexpr int N = 1 << LOGN, T = N / 16, per = kRowThreads / T;
-  const int sub = threadIdx.x / T, tt = threadIdx.x - sub * T;
-  const int gr = blockIdx.x * per + sub;
-  const bool active = gr < planes * p.Fr;
-  const int row = gr % p.Fr, pl = gr / p.Fr;
-  float2 *s = fsm + sub * (N + N / 16);
+  constexpr int N = 1 << LOGN, T = N / 16, per = row_threads(N) / T;
   const ConvGeom &g = p.g;
+  const int sub = threadIdx.x / T, tt = threadIdx.x - sub * T;
+  const int held = p.top + p.bottom;
+  int gr = blockIdx.x * per + sub;
+  const bool image = gr < planes * held;
+  if (!image) gr -= planes * held;
+  const bool active = image || gr < fplanes * g.R;
+  const int per_plane = image ? held : g.R;
+  const int pl = gr / per_plane, q = gr - pl * per_plane;
+  const int row = image && q >= p.top ? p.Fr - held + q : q;  // grid row, or filter row
+  float2 *s = fsm + sub * (N + N / 16);
   float2 v[16];
-  if (SRC == 0) {
-    int ip = 0, fp;
-    if (active) plane_pair(g, pl, 0, &ip, &fp);
-    const float *xp = src + (size_t)ip * g.H * g.W;
-    const int sr = active ? expand_index(row, g.H, p.Fr, g.border) : -1;
+  if (image) {
+    int ip, fp;
+    plane_pair(g, pl, 0, &ip, &fp);
+    const float *xp = x + (size_t)ip * g.H * g.W;
+    const int sr = expand_index(row, g.H, p.Fr, g.border);
     // positions inside the field map to themselves: one 8-byte load per pair
     // (an 8-byte aligned plane of even width keeps every row aligned); the
     // border positions take the expansion rule
@@ -276,96 +308,114 @@ __global__ void __launch_bounds__(kRowThreads, 4)
       }
     }
   } else {
-    const float *fp = src + (size_t)pl * g.R * g.S;
+    const float *fp = f + ((size_t)pl * g.R + row) * g.S;
     const bool conv = g.orient == CCT_CONVOLUTION;
-    const int r = active ? filter_index(row, (g.R - 1) / 2, g.R, p.Fr, conv) : -1;
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
       const int n = tt + m * T;
       float e[2] = {0.0f, 0.0f};
-      if (r >= 0) {
+      if (active) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           const int c = filter_index(2 * n + k, (g.S - 1) / 2, g.S, p.Fc, conv);
-          if (c >= 0) e[k] = __ldg(fp + (size_t)r * g.S + c);
+          if (c >= 0) e[k] = __ldg(fp + c);
         }
       }
       v[m] = make_float2(e[0], e[1]);
     }
   }
-  fft_passes<LOGN, false>(s, v, tt, p.tw_n);
+  fft_regs<LOGN, false, false>(s, v, tt, p.tw_n);
+  if (LOGN > 4) __syncthreads();  // the last exchange is read
+#pragma unroll
+  for (int m = 0; m < 16; ++m) s[pad16(tt + m * T)] = v[m];
+  __syncthreads();
   if (!active) return;
   // X[k] = E[k] + W^k O[k], E = (Z[k] + conj Z[N-k]) / 2, O = (Z[k] - conj Z[N-k]) / 2i,
   // W = exp(-2 pi i / Fc), k = 0..N
-  float2 *out = spec + (size_t)pl * p.Fr * p.ld;
-  for (int k = tt; k <= N; k += T) {
-    const float2 zk = s[pad16(k == N ? 0 : k)], zn = conjf2(s[pad16(k == 0 ? 0 : N - k)]);
+  const int nr = image ? p.Fr : g.R;
+  float2 *out = (image ? spec : rows) + (size_t)pl * nr * p.ld;
+  auto split = [&](int k, float2 zk, float2 zn) {
     const float2 e = make_float2(0.5f * (zk.x + zn.x), 0.5f * (zk.y + zn.y));
     const float2 dd = make_float2(0.5f * (zk.x - zn.x), 0.5f * (zk.y - zn.y));
     const float2 o = make_float2(dd.y, -dd.x);  // dd / i
-    out[spec_index(row, k, p.Fr)] = cadd(e, cmul(__ldg(p.tw_2n + k), o));
+    out[spec_index(row, k, nr)] = cadd(e, cmul(__ldg(p.tw_2n + k), o));
+  };
+#pragma unroll
+  for (int m = 0; m < 16; ++m) {
+    const int k = tt + m * T;
+    split(k, v[m], conjf2(s[pad16(k == 0 ? 0 : N - k)]));
   }
+  if (tt == 0) split(N, v[0], conjf2(v[0]));
 }
 
-// Column pass over blockDim/T spectrum columns per CTA (c fastest across
-// threads, so each warp reads 32-byte row segments).
-// MODE 0: forward FFT, times G[fplane], inverse FFT, in place in spec.
-// MODE 1: forward FFT and scaling by p.scale (a filter's spectrum).
+// Column pass over col_width spectrum columns per CTA (c fastest across
+// threads, so each warp reads 32-byte row segments).  Bound: instruction issue
+// and shared-memory exchanges of one wave of CTAs (2048 rows), their latency
+// below that.  With 512 threads for every length, a 512-row grid had 17 CTAs
+// whose 16 columns shared two bank offsets: 35 us for that pass alone, 4 now.
+// MODE 0: forward FFT, times G[fplane], inverse FFT, in place in spec: rows that
+//         hold the field and its border in, rows of the result out.
+// MODE 1: forward FFT and scaling by p.scale of the filters' rows, into spec.
 template <int MODE, int LOGR>
-__global__ void __launch_bounds__(kColThreads, 2)
-    fft_cols(FftParams p, float2 *__restrict__ spec, const float2 *__restrict__ G, int planes) {
+__global__ void __launch_bounds__(col_width(1 << LOGR) * (1 << LOGR) / 16,
+                                  1024 / (col_width(1 << LOGR) * (1 << LOGR) / 16))
+    fft_cols(FftParams p, float2 *__restrict__ spec, const float2 *__restrict__ G) {
   extern __shared__ __align__(16) float2 fsm[];
   grid_dependency_wait();  // launched with programmatic serialisation
   allow_dependent_launch();
-  constexpr int Fr = 1 << LOGR, T = Fr / 16, CW = kColThreads / T;
+  constexpr int Fr = 1 << LOGR, T = Fr / 16, CW = col_width(Fr);
   const int ncol = p.Fc / 2 + 1;
   const int cblocks = (ncol + CW - 1) / CW;
   const int pl = blockIdx.x / cblocks, c0 = (blockIdx.x - pl * cblocks) * CW;
   const int c = threadIdx.x % CW, tt = threadIdx.x / CW, col = c0 + c;
   const bool active = col < ncol;
-  // column stride = 8 (mod 16) complex: the CW columns a warp touches fall
-  // on alternate halves of the banks
   float2 *s = fsm + c * col_stride(Fr);
   float2 *sp = spec + (size_t)pl * Fr * p.ld + spec_index(0, col, Fr);  // row r at sp[4 r]
   float2 v[16];
+  if (MODE == 0) {
 #pragma unroll
-  for (int m = 0; m < 16; ++m) v[m] = active ? sp[(size_t)(tt + m * T) * 4] : make_float2(0.0f, 0.0f);
-  fft_passes<LOGR, false>(s, v, tt, p.tw_r);
+    for (int m = 0; m < 16; ++m) {
+      const int r = tt + m * T;
+      v[m] = active && (r < p.top || r >= Fr - p.bottom) ? sp[(size_t)r * 4] : make_float2(0.0f, 0.0f);
+    }
+  } else {
+    const ConvGeom &g = p.g;
+    const float2 *rp = G + (size_t)pl * g.R * p.ld + spec_index(0, col, g.R);
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+      const int i = filter_index(tt + m * T, (g.R - 1) / 2, g.R, Fr, g.orient == CCT_CONVOLUTION);
+      v[m] = active && i >= 0 ? __ldg(rp + (size_t)i * 4) : make_float2(0.0f, 0.0f);
+    }
+  }
+  fft_regs<LOGR, false, false>(s, v, tt, p.tw_r);
   if (MODE == 0) {
     int ip, fp;
     plane_pair(p.g, pl, 0, &ip, &fp);
     const float2 *gp = G + (size_t)fp * Fr * p.ld + spec_index(0, col, Fr);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int r = tt + m * T;
-      v[m] = active ? cmul(s[pad16(r)], __ldg(gp + (size_t)r * 4)) : make_float2(0.0f, 0.0f);
-    }
-    fft_passes<LOGR, true>(s, v, tt, p.tw_r);
+    for (int m = 0; m < 16; ++m)
+      v[m] = active ? cmul(v[m], __ldg(gp + (size_t)(tt + m * T) * 4)) : make_float2(0.0f, 0.0f);
+    fft_regs<LOGR, true, true>(s, v, tt, p.tw_r);
     if (!active) return;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int r = tt + m * T;
-      sp[(size_t)r * 4] = s[pad16(r)];
-    }
+    for (int m = 0; m < 16; ++m)
+      if (tt + m * T < p.g.OH) sp[(size_t)(tt + m * T) * 4] = v[m];
   } else {
     if (!active) return;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int r = tt + m * T;
-      sp[(size_t)r * 4] = cscale(s[pad16(r)], p.scale);
-    }
+    for (int m = 0; m < 16; ++m) sp[(size_t)(tt + m * T) * 4] = cscale(v[m], p.scale);
   }
 }
 
 // Inverse row pass: half-spectrum rows -> real rows, trimmed to the output.
 template <int LOGN>
-__global__ void __launch_bounds__(kRowThreads, 4)
+__global__ void __launch_bounds__(row_threads(1 << LOGN), 1024 / row_threads(1 << LOGN))
     fft_rows_c2r(FftParams p, const float2 *__restrict__ spec, float *__restrict__ y, int planes) {
   extern __shared__ __align__(16) float2 fsm[];
   grid_dependency_wait();  // launched with programmatic serialisation
   allow_dependent_launch();
   const ConvGeom &g = p.g;
-  constexpr int N = 1 << LOGN, T = N / 16, per = kRowThreads / T;
+  constexpr int N = 1 << LOGN, T = N / 16, per = row_threads(N) / T;
   const int sub = threadIdx.x / T, tt = threadIdx.x - sub * T;
   const int gr = blockIdx.x * per + sub;
   const bool active = gr < planes * g.OH;
@@ -387,24 +437,24 @@ __global__ void __launch_bounds__(kRowThreads, 4)
     }
     v[m] = z;
   }
-  fft_passes<LOGN, true>(s, v, tt, p.tw_n);
+  fft_regs<LOGN, true, false>(s, v, tt, p.tw_n);
   if (!active) return;
   float *yr = y + ((size_t)pl * g.OH + row) * g.OW;
-  const bool relu = (g.flags & CCT_FLAG_RELU) != 0;
-  if ((g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0) {
-    // an aligned field of even width keeps every output row 8-byte aligned:
-    // one pair per store
-    float2 *yr2 = reinterpret_cast<float2 *>(yr);
-    for (int j = tt; j < g.OW / 2; j += T) {
-      float2 z = s[pad16(j)];
-      if (relu) z = make_float2(fmaxf(z.x, 0.0f), fmaxf(z.y, 0.0f));
-      yr2[j] = z;
-    }
-  } else {
-    for (int j = tt; j < g.OW; j += T) {
-      const float2 z = s[pad16(j >> 1)];
-      const float o = (j & 1) ? z.y : z.x;
-      yr[j] = relu ? fmaxf(o, 0.0f) : o;
+  if ((g.flags & CCT_FLAG_RELU) != 0) {
+#pragma unroll
+    for (int m = 0; m < 16; ++m) v[m] = make_float2(fmaxf(v[m].x, 0.0f), fmaxf(v[m].y, 0.0f));
+  }
+  // an aligned field of even width keeps every output row 8-byte aligned: one
+  // pair per store
+  const bool pairs = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+#pragma unroll
+  for (int m = 0; m < 16; ++m) {
+    const int j = tt + m * T;
+    if (pairs) {
+      if (2 * j < g.OW) reinterpret_cast<float2 *>(yr)[j] = v[m];
+    } else {
+      if (2 * j < g.OW) yr[2 * j] = v[m].x;
+      if (2 * j + 1 < g.OW) yr[2 * j + 1] = v[m].y;
     }
   }
 }
@@ -488,6 +538,11 @@ bool fft_plan(const ConvGeom &g, FftParams *out) {
   p.scale = 1.0f / ((float)p.Fr * (float)(p.Fc / 2));
   p.spec_elems = (size_t)g.pout * p.Fr * p.ld;
   p.filter_elems = (size_t)g.pf * p.Fr * p.ld;
+  p.row_elems = (size_t)g.pf * g.R * p.ld;
+  // a grid larger than the field holds the apron below it and, wrapped, above
+  const bool apron = g.border != CCT_BORDER_ZERO && p.Fr > g.H;
+  p.top = g.H + (apron ? hr : 0);
+  p.bottom = apron ? hr : 0;
   p.tw_elems = (size_t)(p.Fc / 2) + p.Fr + (p.Fc / 2 + 1);
   *out = p;
   return true;
@@ -571,13 +626,15 @@ void fft_static_spectrum(const FftParams &p, const float *host_filter, std::vect
 
 template <int MODE, int L>
 int launch_cols_t(const FftParams &p, float2 *spec, const float2 *G, int planes, cudaStream_t st) {
-  constexpr int Fr = 1 << L, cw = kColThreads / (Fr / 16);
+  constexpr int Fr = 1 << L, cw = col_width(Fr);
   const size_t smem = sizeof(float2) * (size_t)cw * col_stride(Fr);
   int rc = set_smem(fft_cols<MODE, L>, smem);
   if (rc) return rc;
   const int cblocks = (p.Fc / 2 + 1 + cw - 1) / cw;
-  return launch_pdl(fft_cols<MODE, L>, dim3(cblocks * planes), dim3(kColThreads), smem, st, "fft_cols launch", p,
-                    spec, G, planes);
+  rc = launch_pdl(fft_cols<MODE, L>, dim3(cblocks * planes), dim3(cw * Fr / 16), smem, st, "fft_cols launch", p, spec,
+                  G);
+  if (!rc) count_launches(1);
+  return rc;
 }
 
 template <int MODE>
@@ -586,56 +643,51 @@ int launch_cols(const FftParams &p, float2 *spec, const float2 *G, int planes, c
   return CCT_OK;
 }
 
-// Rows per CTA and shared memory of the row passes.
-void row_shape(const FftParams &p, int rows, int *per, int *blocks, size_t *smem) {
-  const int N = p.Fc / 2, T = N / 16;
-  *per = kRowThreads / T;
-  *blocks = (rows + *per - 1) / *per;
-  *smem = sizeof(float2) * (size_t)(*per) * (N + N / 16);
-}
-
-template <int SRC, int L>
-int launch_r2c_t(const FftParams &p, const float *src, float2 *spec, int planes, cudaStream_t st) {
-  int per, blocks;
-  size_t smem;
-  row_shape(p, p.Fr * planes, &per, &blocks, &smem);
-  int rc = set_smem(fft_rows_r2c<SRC, L>, smem);
-  if (rc) return rc;
-  return launch_pdl(fft_rows_r2c<SRC, L>, dim3(blocks), dim3(kRowThreads), smem, st, "fft_rows_r2c launch", p,
-                    src, spec, planes);
+// CTAs and shared memory of a row pass over `rows` sequences of N points.
+template <int L>
+void row_shape(long long rows, unsigned *blocks, size_t *smem) {
+  constexpr int N = 1 << L, per = row_threads(N) / (N / 16);
+  *blocks = (unsigned)((rows + per - 1) / per);
+  *smem = sizeof(float2) * (size_t)per * (N + N / 16);
 }
 
 template <int L>
-int launch_c2r_t(const FftParams &p, const float2 *spec, float *y, int planes, cudaStream_t st) {
-  int per, blocks;
+int launch_r2c_t(const FftParams &p, const float *x, const float *f, float2 *spec, float2 *rows, cudaStream_t st) {
+  const int planes = p.g.pout, fplanes = f ? p.g.pf : 0;
+  unsigned blocks;
   size_t smem;
-  row_shape(p, p.g.OH * planes, &per, &blocks, &smem);
+  row_shape<L>((long long)planes * (p.top + p.bottom) + (long long)fplanes * p.g.R, &blocks, &smem);
+  int rc = set_smem(fft_rows_r2c<L>, smem);
+  if (rc) return rc;
+  rc = launch_pdl(fft_rows_r2c<L>, dim3(blocks), dim3(row_threads(1 << L)), smem, st, "fft_rows_r2c launch", p, x, f,
+                  spec, rows, planes, fplanes);
+  if (!rc) count_launches(1);
+  return rc;
+}
+
+template <int L>
+int launch_c2r_t(const FftParams &p, const float2 *spec, float *y, cudaStream_t st) {
+  const int planes = p.g.pout;
+  unsigned blocks;
+  size_t smem;
+  row_shape<L>((long long)planes * p.g.OH, &blocks, &smem);
   int rc = set_smem(fft_rows_c2r<L>, smem);
   if (rc) return rc;
-  return launch_pdl(fft_rows_c2r<L>, dim3(blocks), dim3(kRowThreads), smem, st, "fft_rows_c2r launch", p, spec,
-                    y, planes);
+  rc = launch_pdl(fft_rows_c2r<L>, dim3(blocks), dim3(row_threads(1 << L)), smem, st, "fft_rows_c2r launch", p, spec, y,
+                  planes);
+  if (!rc) count_launches(1);
+  return rc;
 }
 
-int launch_fft_filter_spectrum(const FftParams &p, const float *f, float2 *G, cudaStream_t st) {
-  const int planes = p.g.pf;
+int launch_fft_conv(const FftParams &p, const float *x, const float *f, float2 *rows, float2 *G, float2 *spec,
+                    float *y, cudaStream_t st) {
   int rc = CCT_OK;
-  CCT_FFT_LOG_SWITCH(p.logN, rc = (launch_r2c_t<1, L>(p, f, G, planes, st)))
-  if (!rc) rc = launch_cols<1>(p, G, nullptr, planes, st);
+  CCT_FFT_LOG_SWITCH(p.logN, rc = (launch_r2c_t<L>(p, x, f, spec, rows, st)))
+  if (!rc && f) rc = launch_cols<1>(p, G, rows, p.g.pf, st);
+  if (!rc) rc = launch_cols<0>(p, spec, G, p.g.pout, st);
   if (rc) return rc;
-  count_launches(2);
-  return check_cuda(cudaGetLastError(), "fft filter spectrum launch");
-}
-
-int launch_fft_conv(const FftParams &p, const float *x, const float2 *G, float2 *spec, float *y,
-                    cudaStream_t st) {
-  const int planes = p.g.pout;
-  int rc = CCT_OK;
-  CCT_FFT_LOG_SWITCH(p.logN, rc = (launch_r2c_t<0, L>(p, x, spec, planes, st)))
-  if (!rc) rc = launch_cols<0>(p, spec, G, planes, st);
+  CCT_FFT_LOG_SWITCH(p.logN, rc = (launch_c2r_t<L>(p, spec, y, st)))
   if (rc) return rc;
-  CCT_FFT_LOG_SWITCH(p.logN, rc = (launch_c2r_t<L>(p, spec, y, planes, st)))
-  if (rc) return rc;
-  count_launches(3);
   return check_cuda(cudaGetLastError(), "fft convolution launch");
 }
 
