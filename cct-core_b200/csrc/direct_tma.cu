@@ -1,6 +1,6 @@
 // Memory-bound direct convolution with TMA halo-tile staging.
 //
-// Persistent CTAs walk 64x128 output tiles; thread 0 keeps kStages tiles in
+// Persistent CTAs walk their output tiles; a loading lane keeps kStages tiles in
 // flight with 3-D TMA loads (cols, rows, plane) completing on mbarriers, so
 // HBM reads overlap the stencil arithmetic.  Zero-fill borders (Zero, Full,
 // and Valid, which never reads outside for kept outputs) come for free from
@@ -15,21 +15,38 @@
 #include "cct_internal.h"
 #include "sm100_util.cuh"
 #include "tile_common.cuh"
+#include "tile_ring.cuh"
 
 namespace cct {
 namespace {
 
 constexpr int kThreads = 256;
-// 64 x 128 output tiles, a thread owning 4 columns x 8 rows: each staged row
-// feeds up to 8 output rows, so the loads, tile bookkeeping and barrier per
-// output are half those of 64 x 64 tiles with 4 rows per thread (0.77 of the
-// copy bandwidth against 0.72); two stages of 38 KB, two CTAs per SM.
-constexpr int kTW = 64, kTH = 128, kU = 4, kV = 8, kTX = 16;
+// 128 x 64 or 64 x 128 output tiles (columns x rows), a thread owning 4 columns
+// x 8 rows: each staged row feeds up to 8 output rows, so the loads, tile
+// bookkeeping and hand-off per output are half those of 64 x 64 tiles with 4 rows
+// per thread (0.77 of the copy bandwidth against 0.72); two stages of 38 KB, two
+// CTAs per SM.  The form that covers the output with less padding is taken, the
+// wide one on a tie (its rows are 512 contiguous bytes: 3x3 on 1024 planes of
+// 256x256 101 us against 104; 64x128 fields 14 against 19, 128x64 ones 21
+// against 15).
+constexpr int kU = 4, kV = 8;
+template <bool WIDE>
+struct TileShape {
+  static constexpr int TW = WIDE ? 128 : 64, TH = WIDE ? 64 : 128, TX = TW / kU;
+};
+// Outputs computed with padding, per output plane.
+template <bool WIDE>
+long long padded(int OH, int OW) {
+  using W = TileShape<WIDE>;
+  return (long long)((OW + W::TW - 1) / W::TW) * W::TW * ((OH + W::TH - 1) / W::TH) * W::TH;
+}
+bool wide_tiles(int OH, int OW) { return padded<true>(OH, OW) <= padded<false>(OH, OW); }
 constexpr int kStages = 2;
 constexpr int kCtasPerSm = 2;
 
-template <int R, int S, int OFF>
+template <int R, int S, int OFF, bool WIDE>
 struct TmaTile {
+  static constexpr int kTW = TileShape<WIDE>::TW, kTH = TileShape<WIDE>::TH;
   static constexpr int IN_ROWS = kTH + R - 1;
   static constexpr int BOX_C = (kTW + S - 1 + OFF + 3) & ~3;
   static constexpr int STAGE = ((IN_ROWS * BOX_C) + 31) & ~31;  // floats, 128-byte multiple
@@ -37,25 +54,29 @@ struct TmaTile {
   static constexpr size_t SMEM = (size_t)kStages * STAGE * 4;
 };
 
-template <int R, int S, int OFF>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+// A loading warp of its own and a ring without CTA barriers, where the 112
+// registers a thread that leaves are enough.  7x7 keeps 49 weights and spills
+// with it (1024 planes of 256x256: 208 us, 166 with thread 0 loading between
+// two barriers per tile); 5x5 goes from 110 to 104.
+constexpr bool own_loader(int R) { return R < 7; }
+constexpr int tma_threads(int R) { return own_loader(R) ? kThreads + 32 : kThreads; }
+
+template <int R, int S, int OFF, bool WIDE>
+__global__ void __launch_bounds__(tma_threads(R), kCtasPerSm)
     direct_tma_kernel(const __grid_constant__ CUtensorMap xmap, ConvGeom g,
                       const float *__restrict__ f, float *__restrict__ y, int tiles_x,
                       int tiles_y, int total, unsigned *err) {
-  using T = TmaTile<R, S, OFF>;
+  using T = TmaTile<R, S, OFF, WIDE>;
+  constexpr int kTW = T::kTW, kTH = T::kTH, kTX = TileShape<WIDE>::TX;
   constexpr int E = (kU - 1) + S;
   constexpr int E4 = (OFF + E + 3) / 4;
   extern __shared__ __align__(128) float smem[];
-  __shared__ __align__(8) uint64_t full[kStages];
+  __shared__ TileRing<kStages, kThreads / 32> ring;
   __shared__ int timed_out;
 
   const int tid = threadIdx.x;
-  const int tx = tid % kTX, ty = tid / kTX;
-  if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
-    timed_out = 0;
-    fence_barrier_init();
-  }
+  ring.init();
+  if (tid == 0) timed_out = 0;
   __syncthreads();
   grid_dependency_wait();  // launched with programmatic serialisation: global memory only after this
   allow_dependent_launch();  // persistent: every CTA is resident already
@@ -66,23 +87,26 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     tyi = q % tiles_y;
     o = q / tiles_y;
   };
-  auto issue = [&](int i, int s) {
+  auto load = [&](int i, int s, uint64_t *full) {
     int o, tyi, txi, ip, fp;
     decode(i, o, tyi, txi);
     plane_pair(g, o, 0, &ip, &fp);
     const int org_r = tyi * kTH - g.low_r;
     const int start_c = txi * kTW - g.low_c - OFF;  // multiple of 4
-    mbar_arrive_expect_tx(&full[s], T::BYTES);
-    tma_load_3d(smem + s * T::STAGE, &xmap, &full[s], start_c, org_r, ip);
+    mbar_arrive_expect_tx(full, T::BYTES);
+    tma_load_3d(smem + s * T::STAGE, &xmap, full, start_c, org_r, ip);
   };
-
-  if (tid == 0) {
+  if (own_loader(R) && tid >= kThreads) {
+    if (tid == kThreads) ring.produce(total, err, load);
+    return;
+  }
+  if (!own_loader(R) && tid == 0)
     for (int k = 0; k < kStages; ++k) {
       const int i = blockIdx.x + k * gridDim.x;
-      if (i < total) issue(i, k);
+      if (i < total) load(i, k, &ring.full[k]);
     }
-  }
 
+  const int tx = tid % kTX, ty = tid / kTX;
   const bool conv = g.orient == CCT_CONVOLUTION;
   const bool relu = (g.flags & CCT_FLAG_RELU) != 0;
   const bool vec_store = (g.OW & 3) == 0;
@@ -93,7 +117,6 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
   int j = 0;
   for (int i = blockIdx.x; i < total; i += gridDim.x, ++j) {
     const int s = j % kStages;
-    const uint32_t parity = (uint32_t)((j / kStages) & 1);
     int o, tyi, txi, ip, fp;
     decode(i, o, tyi, txi);
     plane_pair(g, o, 0, &ip, &fp);
@@ -106,17 +129,19 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
           w[r][c] = __ldg(fs + (conv ? (R - 1 - r) * S + (S - 1 - c) : r * S + c));
       cur_fp = fp;
     }
-    if (!mbar_wait(&full[s], parity, err)) timed_out = 1;
-    __syncthreads();
-    if (timed_out) {
-      // Give the copies still in flight a bounded chance to land, then leave.
-      if (tid == 0)
-        for (int k = 1; k < kStages; ++k) {
-          const int jj = j + k;
-          if (blockIdx.x + jj * gridDim.x < total)
-            mbar_wait(&full[jj % kStages], (uint32_t)((jj / kStages) & 1), err);
-        }
-      return;
+    if constexpr (own_loader(R)) {
+      if (!ring.wait_full(j, err)) return;
+    } else {
+      if (!mbar_wait(&ring.full[s], (uint32_t)((j / kStages) & 1), err)) timed_out = 1;
+      __syncthreads();
+      if (timed_out) {
+        // Give the copies still in flight a bounded chance to land, then leave.
+        if (tid == 0)
+          for (int k = j + 1; k < j + kStages; ++k)
+            if (blockIdx.x + k * gridDim.x < total)
+              mbar_wait(&ring.full[k % kStages], (uint32_t)((k / kStages) & 1), err);
+        return;
+      }
     }
 
     const float *base = smem + s * T::STAGE + (ty * kV) * T::BOX_C + tx * kU;
@@ -150,6 +175,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         }
       }
     }
+    if constexpr (own_loader(R)) ring.release(s);  // this warp is done with the stage
 
     float *ys = y + (size_t)o * opage;
     const int col0 = txi * kTW + tx * kU;
@@ -169,13 +195,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
           if (col0 + u < g.OW) dst[u] = out[u];
       }
     }
-
-    __syncthreads();  // every thread is done with stage s
-    if (tid == 0) {
+    if constexpr (!own_loader(R)) {
+      __syncthreads();  // every thread is done with stage s
       const int next = i + kStages * gridDim.x;
-      if (next < total) {
+      if (tid == 0 && next < total) {
         fence_proxy_async_smem();
-        issue(next, s);
+        load(next, s, &ring.full[s]);
       }
     }
   }
@@ -205,7 +230,7 @@ EncodeFn encode_fn() {
 std::mutex g_attr_mu;
 std::unordered_map<uint64_t, int> g_resident;
 
-int resident_ctas(const void *func, size_t bytes, int *ctas) {
+int resident_ctas(const void *func, int threads, size_t bytes, int *ctas) {
   int dev = 0;
   cudaGetDevice(&dev);
   const uint64_t key = reinterpret_cast<uint64_t>(func) ^ ((uint64_t)dev << 56);
@@ -221,29 +246,30 @@ int resident_ctas(const void *func, size_t bytes, int *ctas) {
   if (rc) return rc;
   int sms = 148, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, kThreads, bytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, bytes);
   *ctas = g_resident[key] = std::max(per_sm, 1) * sms;
   return CCT_OK;
 }
 
-template <int R, int OFF>
+template <int R, int OFF, bool WIDE>
 int launch_tma(const ConvGeom &g, const float *x, const float *f, float *y, cudaStream_t st,
                unsigned *err) {
-  using T = TmaTile<R, R, OFF>;
+  using T = TmaTile<R, R, OFF, WIDE>;
+  constexpr int kTW = T::kTW, kTH = T::kTH;
   CUtensorMap map;
   int rc = encode_tensor_map_3d(&map, x, g.W, g.H, g.pin, T::BOX_C, T::IN_ROWS);
   if (rc) return rc;
   const int tiles_x = (g.OW + kTW - 1) / kTW, tiles_y = (g.OH + kTH - 1) / kTH;
   const long long total = (long long)tiles_x * tiles_y * g.pout;
   if (total > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "direct convolution grid too large");
-  auto kern = direct_tma_kernel<R, R, OFF>;
+  auto kern = direct_tma_kernel<R, R, OFF, WIDE>;
   // persistent CTAs: as many as are resident at once (registers and shared
   // memory decide), so no CTA waits for another to finish
   int resident = 0;
-  rc = resident_ctas((const void *)kern, T::SMEM, &resident);
+  rc = resident_ctas((const void *)kern, tma_threads(R), T::SMEM, &resident);
   if (rc) return rc;
   const int grid = (int)std::min<long long>(total, resident);
-  const int rc2 = launch_pdl(kern, dim3(grid), dim3(kThreads), T::SMEM, st, "direct_tma_kernel launch", map, g, f,
+  const int rc2 = launch_pdl(kern, dim3(grid), dim3(tma_threads(R)), T::SMEM, st, "direct_tma_kernel launch", map, g, f,
                              y, tiles_x, tiles_y, (int)total, err);
   if (!rc2) count_launches(1);
   return rc2;
@@ -298,19 +324,22 @@ bool direct_tma_supported(const ConvGeom &g, const float *x) {
   if (g.R != g.S || (g.R != 1 && g.R != 3 && g.R != 5 && g.R != 7)) return false;
   if ((g.W & 3) != 0) return false;
   if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
-  // Fewer than 96 of these 64 x 128 tiles leave most SMs idle, and a field of
-  // at most 64 rows half of each tile: the direct stencils' smaller tiles are
-  // faster there (us, 5x5: one plane of 256x256 4.0 / 2.4, eight 4.2 / 3.7,
-  // sixteen 4.2 / 5.3; 512 planes of 60x64 9.1 / 7.4).
-  const long long tiles = (long long)((g.OW + kTW - 1) / kTW) * ((g.OH + kTH - 1) / kTH) * g.pout;
-  return tiles >= 96 && g.OH > 64;
+  // Fewer than 96 of these tiles leave most SMs idle, and a field that fills
+  // less than half of its tiles wastes the rest: the direct stencils' smaller
+  // tiles are faster there (us, 5x5: one plane of 256x256 4.0 / 2.4, eight 4.2 /
+  // 3.7, sixteen 4.2 / 5.3; 2048 planes of 60x64 27.3 / 25.4).
+  const long long outs = padded<true>(g.OH, g.OW) < padded<false>(g.OH, g.OW) ? padded<true>(g.OH, g.OW)
+                                                                               : padded<false>(g.OH, g.OW);
+  return outs / (64 * 128) * g.pout >= 96 && outs < 2LL * g.OH * g.OW;
 }
 
 int launch_direct_tma(const ConvGeom &g, const float *x, const float *f, float *y,
                       cudaStream_t st, unsigned *err) {
   const int off = ((g.low_c % 4) == 0) ? 0 : 4 - (g.low_c % 4);  // (-low_c) mod 4
 #define CCT_TMA_CASE(RR, OO) \
-  if (g.R == RR && off == OO) return launch_tma<RR, OO>(g, x, f, y, st, err);
+  if (g.R == RR && off == OO)   \
+    return wide_tiles(g.OH, g.OW) ? launch_tma<RR, OO, true>(g, x, f, y, st, err) \
+                                  : launch_tma<RR, OO, false>(g, x, f, y, st, err);
   CCT_TMA_CASE(1, 0)
   CCT_TMA_CASE(3, 0) CCT_TMA_CASE(3, 2) CCT_TMA_CASE(3, 3)
   CCT_TMA_CASE(5, 0) CCT_TMA_CASE(5, 2)

@@ -124,3 +124,24 @@ def test_up_bank(mode, rows, cols, R, step):
                                                        (16, 64, 0, 1, "zero")])
 def test_widest(S, rows, cols, planes, R, border):
     _check(rows, cols, R, S, border, O.CONV if S % 4 == 1 else O.XCORR, planes=planes)
+
+
+# the TMA stencils' two tile forms (64 x 128 and 128 x 64), with last tiles of one
+# row or 4 columns and more tiles than the persistent grid's two stages hold
+@pytest.mark.parametrize("border", ["zero", "valid", "full"])
+@pytest.mark.parametrize("R", [1, 3, 5, 7])
+@pytest.mark.parametrize("planes,rows,cols", [(400, 129, 64), (1300, 65, 132), (330, 64, 128), (700, 128, 68)])
+def test_tma_tiles(planes, rows, cols, R, border):
+    _check(rows, cols, R, R, border, O.CONV, planes=planes)
+
+
+@pytest.mark.parametrize("rl,cl", [(1, 9), (3, 5), (5, 3), (7, 7), (9, 1)])
+@pytest.mark.parametrize("planes,rows,cols", [(400, 129, 64), (1300, 65, 132), (5, 30, 20)])
+def test_separable_tma_tiles(planes, rows, cols, rl, cl):
+    rng = np.random.default_rng(rows + rl)
+    x = rng.uniform(-1, 1, (planes, rows, cols)).astype(np.float32)
+    rf, cf = rng.uniform(-1, 1, rl).astype(np.float32), rng.uniform(-1, 1, cl).astype(np.float32)
+    import cctconv as C
+    y = C.crossCorrelateSeparable(torch.from_numpy(x).cuda(), torch.from_numpy(rf).cuda(), torch.from_numpy(cf).cuda(),
+                                  C.BorderZero)
+    assert bitwise_equal(y.cpu().numpy(), O.separable(x, rf, cf, O.ZERO, O.XCORR))
