@@ -3,14 +3,16 @@
 // Each output is a fused multiply-add chain from 0 over the 1-D filter taps,
 // the order of the reference's `sum += localImage[..] * filter` loop.
 // Short filters run both passes fused per output tile: under BorderZero on
-// fields whose width is a multiple of 4 floats the halo tiles arrive by TMA
-// (separable_tma), otherwise threads stage them (separable_fused_t /
-// separable_fused); long filters run one thread per output per pass, through
-// a scratch field.
+// large fields whose width is a multiple of 4 floats the halo tiles arrive by
+// TMA (separable_tma, up to 9 taps), otherwise threads stage them
+// (separable_tile, up to 15 + 31 taps; separable_fused, up to about 33); long
+// filters run one thread per output per pass, through a scratch field.
+#include <algorithm>
 #include <atomic>
 
 #include "cct_internal.h"
 #include "sm100_util.cuh"
+#include "stencil.cuh"
 #include "tile_common.cuh"
 #include "tile_ring.cuh"
 
@@ -128,102 +130,167 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// The same fused tile with the filter lengths fixed at compile time (1, 3,
-// 5, 7 or 9): each thread slides a register window along 8 outputs of a row
-// in the rows pass and down 8 outputs of a column in the columns pass, so a
-// tap costs a multiply-add and not a shared-memory read.
-template <int RL, int CL>
-struct SepTile {
-  static constexpr int hr = (RL - 1) / 2, hc = (CL - 1) / 2, U = 8;
-  // Odd pitches keep both passes free of bank conflicts: in the rows pass a
-  // warp's lanes walk down 32 staged rows of one 8-column block (pitch IC)
-  // and write the intermediate down a column (pitch MP); in the columns pass
-  // lanes walk along a row of the intermediate.
-  static constexpr int IR = kSTH + CL - 1, ICU = kSTW + RL - 1, IC = ICU | 1, MP = kSTW + 1;
-};
+// Row filters of up to 15 taps (compiled), column filters of up to 31, every
+// border and width.  A CTA of 128 threads computes 64 columns x 8 V rows: the
+// halo is staged with the columns mapped once per tile (TileStage), the rows
+// pass slides a register window along 8 columns of a staged row, and the columns
+// pass keeps 4 columns x V rows per thread, so a row-filtered value is read once
+// per V outputs.  Each value is the same fma chain as in the two-pass form.
+// Bound: FP32 issue and staging latency.  The forms it replaces mapped every
+// staged element by the border, and past 9 taps read shared memory per tap:
+// 1080x1920 x3, 7 + 7 clamp 31 us, 720x1280 x3, 15 + 15 35 us; 21.4 and 14.0 here.
+constexpr int kTlThreads = 128, kTlW = 64, kTlMid = kTlW + 4, kTlMaxR = 15, kTlMaxC = 31;
+__host__ __device__ constexpr int tile_pitch(int RL) {
+  const int c = (kTlW + RL - 1 + 3) & ~3;
+  return (c & 7) == 4 ? c : c + 4;  // 4 (mod 8): two rows of a float4 phase on different banks
+}
+inline size_t tile_smem(int RL, int clen, int V) {
+  return sizeof(float) * ((size_t)(8 * V + clen - 1) * (tile_pitch(RL) + kTlMid) + kTlMaxC + 1);
+}
 
-template <int RL, int CL>
-__global__ void __launch_bounds__(kThreads)
-    separable_fused_t(int rows, int cols, const float *__restrict__ x, const float *__restrict__ rf,
-                      const float *__restrict__ cf, int border, int orient, float *__restrict__ y,
-                      int tiles_x, int tiles_y, long long tiles) {
+template <int RL, int V>
+__global__ void __launch_bounds__(kTlThreads, V == 8 ? 5 : 8)
+    separable_tile(int rows, int cols, const float *__restrict__ x, const float *__restrict__ rf,
+                   const float *__restrict__ cf, int clen, int border, int orient, float *__restrict__ y, int tiles_x,
+                   int tiles_y) {
+  constexpr int TH = 8 * V, PITCH = tile_pitch(RL), U = 8, E4 = (U + RL - 1 + 3) / 4;
+  static_assert(4 * E4 + kTlW - U <= PITCH, "a thread's loads stay inside its row");
+  extern __shared__ __align__(16) float sm[];
+  const int IR = TH + clen - 1;
+  float *img = sm, *mid = sm + IR * PITCH, *wc = mid + IR * kTlMid;
   grid_dependency_wait();  // launched with programmatic serialisation: nothing global before this
-  using T = SepTile<RL, CL>;
-  constexpr int IR = T::IR, IC = T::IC, MP = T::MP, U = T::U, hr = T::hr, hc = T::hc, ICU = T::ICU;
-  __shared__ float img[IR * IC];
-  __shared__ float mid[IR * MP];
-  float wr[RL], wc[CL];
   const bool conv = orient == CCT_CONVOLUTION;
+  int bid = blockIdx.x;
+  const int tx_i = bid % tiles_x;
+  bid /= tiles_x;
+  const int ty_i = bid % tiles_y, pl = bid / tiles_y;
+  const int r0 = ty_i * TH, c0 = tx_i * kTlW, out_rows = min(TH, rows - r0), need = out_rows + clen - 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ConvGeom g;  // what the staging reads
+  g.H = rows;
+  g.W = cols;
+  g.border = border;
+  {
+    const TileStage<kTlW + RL - 1, PITCH, kTlThreads, false> stage(g, c0 - (RL - 1) / 2);
+    stage.copy(img, x + (size_t)pl * rows * cols, g, r0 - (clen - 1) / 2, need);
+    cp_async_commit();
+  }
+  float wr[RL];
 #pragma unroll
   for (int k = 0; k < RL; ++k) wr[k] = __ldg(rf + (conv ? RL - 1 - k : k));
+  if (threadIdx.x < clen) wc[threadIdx.x] = __ldg(cf + (conv ? clen - 1 - (int)threadIdx.x : (int)threadIdx.x));
+  cp_async_wait<0>();
+  __syncthreads();
+  {
+    // a float4 phase of 8 lanes covers 4 column blocks x 2 rows
+    const int cb = (lane & 3) | ((lane >> 1) & 4), rsub = ((lane >> 2) & 1) | ((lane >> 3) & 2);
+    for (int r = warp * 4 + rsub; r < need; r += 16) {
+      const float *line = img + r * PITCH + cb * U;
+      float win[4 * E4];
 #pragma unroll
-  for (int k = 0; k < CL; ++k) wc[k] = __ldg(cf + (conv ? CL - 1 - k : k));
-  int bid = blockIdx.x;
-  const int tx = bid % tiles_x;
-  bid /= tiles_x;
-  const int ty = bid % tiles_y, pl = bid / tiles_y;
-  const int r0 = ty * kSTH, c0 = tx * kSTW;
-  const float *xp = x + (size_t)pl * rows * cols;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const bool inside_c = c0 - hr >= 0 && c0 - hr + ICU <= cols;
-  for (int ir = warp; ir < IR; ir += nwarps) {
-    const int sr = border_index(border, r0 - hc + ir, rows);
-    float *dst = img + ir * IC;
-    if (sr < 0) {
-      for (int ic = lane; ic < ICU; ic += 32) dst[ic] = 0.0f;
-    } else if (inside_c) {
-      const float *src = xp + (size_t)sr * cols + (c0 - hr);
-      for (int ic = lane; ic < ICU; ic += 32) dst[ic] = __ldg(src + ic);
-    } else {
-      const float *src = xp + (size_t)sr * cols;
-      for (int ic = lane; ic < ICU; ic += 32) {
-        const int sc = border_index(border, c0 - hr + ic, cols);
-        dst[ic] = sc >= 0 ? __ldg(src + sc) : 0.0f;
+      for (int e = 0; e < E4; ++e) {
+        const float4 q = *reinterpret_cast<const float4 *>(line + 4 * e);
+        win[4 * e + 0] = q.x;
+        win[4 * e + 1] = q.y;
+        win[4 * e + 2] = q.z;
+        win[4 * e + 3] = q.w;
+      }
+      float h[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < RL; ++k) sum = __fmaf_rn(win[u + k], wr[k], sum);
+        h[u] = sum;
+      }
+      float4 *dst = reinterpret_cast<float4 *>(mid + r * kTlMid + cb * U);
+      dst[0] = make_float4(h[0], h[1], h[2], h[3]);
+      dst[1] = make_float4(h[4], h[5], h[6], h[7]);
+    }
+  }
+  __syncthreads();
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[V][4];
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[v][u] = 0.0f;
+  if (ty * V < out_rows) {
+    const float *base = mid + ty * V * kTlMid + tx * 4;
+    for (int tr = 0; tr < V - 1 + clen; ++tr) {
+      const float4 q = *reinterpret_cast<const float4 *>(base + tr * kTlMid);
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int k = tr - v;
+        if (k >= 0 && k < clen) {  // the same for every thread
+          const float w = wc[k];
+          acc[v][0] = __fmaf_rn(q.x, w, acc[v][0]);
+          acc[v][1] = __fmaf_rn(q.y, w, acc[v][1]);
+          acc[v][2] = __fmaf_rn(q.z, w, acc[v][2]);
+          acc[v][3] = __fmaf_rn(q.w, w, acc[v][3]);
+        }
       }
     }
   }
-  __syncthreads();
-  for (int item = threadIdx.x; item < IR * (kSTW / U); item += blockDim.x) {
-    const int jb = item / IR, ir = item - jb * IR, j0 = jb * U;
-    const float *line = img + ir * IC + j0;
-    float win[U + RL - 1];
+  allow_dependent_launch();
+  float *yp = y + (size_t)pl * rows * cols + (size_t)r0 * cols + c0;
+  if ((cols & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+    if (c0 + tx * 4 >= cols) return;
 #pragma unroll
-    for (int k = 0; k < U + RL - 1; ++k) win[k] = line[k];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int k = 0; k < RL; ++k) sum = __fmaf_rn(win[u + k], wr[k], sum);
-      mid[ir * MP + j0 + u] = sum;
-    }
+    for (int v = 0; v < V; ++v)
+      if (ty * V + v < out_rows)
+        *reinterpret_cast<float4 *>(yp + (size_t)(ty * V + v) * cols + tx * 4) =
+            make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+    return;
   }
-  __syncthreads();
-  float *yp = y + (size_t)pl * rows * cols;
-  for (int item = threadIdx.x; item < kSTW * (kSTH / U); item += blockDim.x) {
-    const int j = item % kSTW, i0 = (item / kSTW) * U;
-    const int c = c0 + j;
-    float win[U + CL - 1];
+  // rows that are not 16-byte aligned leave through the image's tile, which the
+  // rows pass has read: a warp stores 32 adjacent values at a time
 #pragma unroll
-    for (int k = 0; k < U + CL - 1; ++k) win[k] = mid[(i0 + k) * MP + j];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int k = 0; k < CL; ++k) sum = __fmaf_rn(win[u + k], wc[k], sum);
-      const int r = r0 + i0 + u;
-      if (r < rows && c < cols) yp[(size_t)r * cols + c] = sum;
-    }
-  }
+  for (int v = 0; v < V; ++v)
+    *reinterpret_cast<float4 *>(img + (ty * V + v) * kTlW + tx * 4) =
+        make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+  __syncwarp();
+  const int w0 = warp * 2 * V;
+  if (w0 < out_rows)
+    store_rows64(yp + (size_t)w0 * cols, cols, img + w0 * kTlW, kTlW, min(2 * V, out_rows - w0), min(kTlW, cols - c0),
+                 lane);
 }
 
-template <int RL, int CL>
-int launch_fused_t(int rows, int cols, const float *x, const float *rf, const float *cf, int border,
-                   int orient, float *y, int tiles_x, int tiles_y, long long tiles, cudaStream_t st) {
-  if (tiles > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "separable: grid too large");
-  const int rc = launch_pdl(separable_fused_t<RL, CL>, dim3((unsigned)tiles), dim3(kThreads), 0, st,
-                            "separable launch", rows, cols, x, rf, cf, border, orient, y, tiles_x, tiles_y, tiles);
+template <int RL, int V>
+int launch_tile_v(int rows, int cols, int planes, const float *x, const float *rf, const float *cf, int clen,
+                  int border, int orient, float *y, cudaStream_t st, long long min_blocks) {
+  const int tx = (cols + kTlW - 1) / kTlW, ty = (rows + 8 * V - 1) / (8 * V);
+  const long long blocks = (long long)tx * ty * planes;
+  if (blocks < min_blocks) return 1;  // a shorter tile is wanted
+  if (blocks > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "separable: grid too large");
+  const size_t smem = tile_smem(RL, clen, V);
+  if (smem > 48 * 1024) {
+    const int rc = check_cuda(cudaFuncSetAttribute(separable_tile<RL, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem),
+                              "cudaFuncSetAttribute(separable_tile)");
+    if (rc) return rc;
+  }
+  const int rc = launch_pdl(separable_tile<RL, V>, dim3((unsigned)blocks), dim3(kTlThreads), smem, st,
+                            "separable launch", rows, cols, x, rf, cf, clen, border, orient, y, tx, ty);
   if (!rc) count_launches(1);
   return rc;
+}
+
+// The tile form for a row filter of 1, 3, .. 15 taps; tall tiles once they give
+// each of 148 SMs two CTAs.
+int launch_tile(int rows, int cols, int planes, const float *x, const float *rf, int rlen, const float *cf, int clen,
+                int border, int orient, float *y, cudaStream_t st) {
+#define CCT_TILE_CASE(RL)                                                                                          \
+  case RL: {                                                                                                       \
+    const int rc = launch_tile_v<RL, 8>(rows, cols, planes, x, rf, cf, clen, border, orient, y, st, 2 * 148);      \
+    return rc == 1 ? launch_tile_v<RL, 2>(rows, cols, planes, x, rf, cf, clen, border, orient, y, st, 0) : rc;     \
+  }
+  switch (rlen) {
+    CCT_TILE_CASE(1) CCT_TILE_CASE(3) CCT_TILE_CASE(5) CCT_TILE_CASE(7)
+    CCT_TILE_CASE(9) CCT_TILE_CASE(11) CCT_TILE_CASE(13) CCT_TILE_CASE(15)
+    default: return set_error(CCT_ENOTSUP, "separable: row filter of %d taps", rlen);
+  }
+#undef CCT_TILE_CASE
 }
 
 // BorderZero with TMA staging: persistent CTAs walk their output tiles and a
@@ -413,21 +480,6 @@ int launch_tma_small(int rows, int cols, int planes, const float *x, const float
   return -1;
 }
 
-// Compile-time lengths 1, 3, 5, 7, 9 for both filters; -1 if not covered,
-// else the launch status.
-int launch_fused_small(int rows, int cols, const float *x, const float *rf, int rlen, const float *cf,
-                       int clen, int border, int orient, float *y, int tiles_x, int tiles_y, long long tiles,
-                       cudaStream_t st) {
-#define CCT_SEP_C(RL, CL)                                                                                 \
-  if (rlen == RL && clen == CL)                                                                           \
-    return launch_fused_t<RL, CL>(rows, cols, x, rf, cf, border, orient, y, tiles_x, tiles_y, tiles, st);
-#define CCT_SEP_R(RL) CCT_SEP_C(RL, 1) CCT_SEP_C(RL, 3) CCT_SEP_C(RL, 5) CCT_SEP_C(RL, 7) CCT_SEP_C(RL, 9)
-  CCT_SEP_R(1) CCT_SEP_R(3) CCT_SEP_R(5) CCT_SEP_R(7) CCT_SEP_R(9)
-#undef CCT_SEP_R
-#undef CCT_SEP_C
-  return -1;
-}
-
 size_t separable_fused_smem(int rlen, int clen) {
   const size_t IR = kSTH + clen - 1, IC = kSTW + rlen - 1;
   return sizeof(float) * (rlen + clen + IR * IC + IR * kSTW);
@@ -452,14 +504,17 @@ int launch_separable(int rows, int cols, int planes, const float *x, const float
   if (fsmem <= 96 * 1024) {
     const int tiles_x = (cols + kSTW - 1) / kSTW, tiles_y = (rows + kSTH - 1) / kSTH;
     const long long blocks = (long long)tiles_x * tiles_y * planes;
+    // Fewer than 96 TMA tiles leave most SMs idle; the smaller tiles below do not
+    // (us: one plane of 512x512, 5 + 5, 32 tiles 3.4 / 2.7; 768x768, 72 tiles 3.5 /
+    // 3.3; 1024x1024, 128 tiles 3.7 / 4.4).
+    const long long pad = std::min(SepShape<true>::padded(rows, cols), SepShape<false>::padded(rows, cols));
     if (border == CCT_BORDER_ZERO && (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
-        (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+        (reinterpret_cast<uintptr_t>(y) & 15) == 0 && pad / (64 * 128) * planes >= 96) {
       const int rc = launch_tma_small(rows, cols, planes, x, rf, rlen, cf, clen, orient, y, st);
       if (rc >= 0) return rc;
     }
-    const int rc = launch_fused_small(rows, cols, x, rf, rlen, cf, clen, border, orient, y, tiles_x, tiles_y,
-                                      blocks, st);
-    if (rc >= 0) return rc;
+    if (rlen <= kTlMaxR && clen <= kTlMaxC)
+      return launch_tile(rows, cols, planes, x, rf, rlen, cf, clen, border, orient, y, st);
     if (blocks <= 0x7fffffffLL) {
       if (fsmem > 48 * 1024) {
         int rc = check_cuda(cudaFuncSetAttribute(separable_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,

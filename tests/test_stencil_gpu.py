@@ -145,3 +145,19 @@ def test_separable_tma_tiles(planes, rows, cols, rl, cl):
     y = C.crossCorrelateSeparable(torch.from_numpy(x).cuda(), torch.from_numpy(rf).cuda(), torch.from_numpy(cf).cuda(),
                                   C.BorderZero)
     assert bitwise_equal(y.cpu().numpy(), O.separable(x, rf, cf, O.ZERO, O.XCORR))
+
+
+# the separable tile form: tall and short tiles, every compiled row length, column
+# lengths up to its limit and past it, 16- and 4-byte stores, fields smaller than
+# the filters
+@pytest.mark.parametrize("border", ["zero", "clamp", "cyclic"])
+@pytest.mark.parametrize("rl,cl", [(1, 31), (3, 1), (5, 9), (7, 7), (9, 15), (11, 3), (13, 13), (15, 31), (15, 33), (17, 5)])
+@pytest.mark.parametrize("planes,rows,cols", [(160, 65, 130), (2, 17, 65), (1, 6, 5), (3, 64, 72)])
+def test_separable_tiles(planes, rows, cols, rl, cl, border):
+    import cctconv as C
+    rng = np.random.default_rng(rows * 40 + rl)
+    x = rng.uniform(-1, 1, (planes, rows, cols)).astype(np.float32)
+    rf, cf = rng.uniform(-1, 1, rl).astype(np.float32), rng.uniform(-1, 1, cl).astype(np.float32)
+    b = {"zero": C.BorderZero, "clamp": C.BorderClamp, "cyclic": C.BorderCyclic}[border]
+    y = C.convolveSeparable(torch.from_numpy(x).cuda(), torch.from_numpy(rf).cuda(), torch.from_numpy(cf).cuda(), b)
+    assert bitwise_equal(y.cpu().numpy(), O.separable(x, rf, cf, _BORDERS[border], O.CONV))
