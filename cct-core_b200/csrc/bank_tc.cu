@@ -95,25 +95,51 @@ __host__ __device__ constexpr int block_term(int terms, int blk) {
 // Paired taps (banks of at most 32 filters): a chunk of 32-row blocks
 // [0 0 Fh_a Fh_b Fl_a Fl_b] for taps a and b = a + 1 of one filter row, the
 // same 192 rows and MMAs as an unpaired two-term chunk: [Fh_a; Fh_b; Fl_a;
-// Fl_b] x Xh and [0; 0; Fh_a; Fh_b] x Xl.  -1 zero, else (term, which tap).
-__host__ __device__ constexpr int pair_block_term(int blk) { return blk < 2 ? -1 : blk < 4 ? 0 : 1; }
-__host__ __device__ constexpr int pair_block_tap(int blk) { return blk & 1; }
-template <int TERMS, bool PAIR>
+// Fl_b] x Xh and [0; 0; Fh_a; Fh_b] x Xl.
+// Forms of a filter block (BankParams::form).
+//   kPlain     64 filters; big and small sums in separate rows (above)
+//   kPair      32 filters x two taps, rows as above
+//   kWide      128 filters; big and small sums in separate columns
+//   kWidePair  64 filters x two taps, sums as kWide
+// The wide forms need no zero rows: a chunk is each split term's 128 rows, an
+// accumulator is 128 columns of big sums and 128 of small ones (N <= 128), and
+// every MMA's rows are all live: 6 MMAs of N = 128 do 128 x 128 outputs where the
+// plain form's 5 of N = 256 do 64 x 256 (three terms; 3 against 2 for two).
+enum { kPlain = 0, kPair = 1, kWide = 2, kWidePair = 3 };
+__host__ __device__ constexpr bool pairs_taps(int form) { return form == kPair || form == kWidePair; }
+__host__ __device__ constexpr bool wide_form(int form) { return form >= kWide; }
+// Parts of a filter's sum in different rows (warps): big and small, tap a and tap b.
+__host__ __device__ constexpr int form_parts(int form) { return form == kPair ? 4 : form == kWide ? 1 : 2; }
+
+template <int TERMS, bool WIDE>
 struct MmaList;
 template <>
 struct MmaList<2, false> {
   static constexpr int n = 2;
-  __device__ static int arow(int m) { return m == 0 ? 64 : 0; }  // [Fh; Fl], [0; Fh]
+  __device__ static int arow(int m) { return m == 0 ? 64 : 0; }  // [Fh; Fl], [0; Fh] (paired: at tap a's offset)
   __device__ static int bterm(int m) { return m; }               // Xh, Xl
 };
-template <>
-struct MmaList<2, true> : MmaList<2, false> {};  // at tap a's offset
 template <>
 struct MmaList<3, false> {
   static constexpr int n = 5;
   // [Fh; Fm] x Xh, [0; Fh] x Xm, [0; Fh] x Xl, [0; Fl] x Xh, [0; Fm] x Xm
   __device__ static int arow(int m) { return m == 0 ? 64 : m == 3 ? 192 : m == 4 ? 320 : 0; }
   __device__ static int bterm(int m) { return m == 0 || m == 3 ? 0 : m == 2 ? 2 : 1; }
+};
+// Wide: MMA 0 into the big columns, the others into the small ones.
+template <>
+struct MmaList<2, true> {
+  static constexpr int n = 3;
+  // Fh x Xh; Fl x Xh, Fh x Xl
+  __device__ static int arow(int m) { return m == 1 ? 128 : 0; }
+  __device__ static int bterm(int m) { return m == 2 ? 1 : 0; }
+};
+template <>
+struct MmaList<3, true> {
+  static constexpr int n = 6;
+  // Fh x Xh; Fm x Xh, Fl x Xh, Fh x Xm, Fm x Xm, Fh x Xl
+  __device__ static int arow(int m) { return m == 1 || m == 4 ? 128 : m == 2 ? 256 : 0; }
+  __device__ static int bterm(int m) { return m < 3 ? 0 : m < 5 ? 1 : 2; }
 };
 
 struct Bars {
@@ -166,7 +192,7 @@ struct ItemUnits {
   int ts, nu, nst;
   size_t chunk0;
 };
-template <bool PAIR>
+template <int FORM>
 __device__ __forceinline__ ItemUnits item_units(const BankParams &p, const Item &it) {
   ItemUnits r;
   int rows;
@@ -178,7 +204,7 @@ __device__ __forceinline__ ItemUnits item_units(const BankParams &p, const Item 
     rows = p.g.R;
     r.ts = p.g.S;
   }
-  r.nu = rows * (PAIR ? (r.ts + 1) / 2 : r.ts);
+  r.nu = rows * (pairs_taps(FORM) ? (r.ts + 1) / 2 : r.ts);
   r.nst = (r.nu + p.T - 1) / p.T;
   r.chunk0 = (size_t)p.up_choff[it.ph] + (size_t)it.nb * p.NCB * r.nu;
   return r;
@@ -227,6 +253,25 @@ __device__ __forceinline__ void convert_kgroups(const float *src, size_t plane, 
   store_kgroups<TERMS, KG>(v, dst, kg_stride, part_bytes);
 }
 
+// A barrier over the G warps of a group (one warp: none but itself).
+template <int G>
+__device__ __forceinline__ void group_sync(int bar_id) {
+  if (G == 1)
+    __syncwarp();
+  else
+    named_sync(bar_id, 32 * G);
+}
+template <int G>
+__device__ __forceinline__ bool group_sync_or(int bar_id, bool pred) {
+  return G == 1 ? __any_sync(0xffffffffu, pred) != 0 : named_sync_or(bar_id, 32 * G, pred);
+}
+// Where a warp's lane quarter stands: its group, and its part in it.
+template <int FORM>
+__device__ __forceinline__ void group_of(int quarter, int half, int &grp, int &part) {
+  grp = FORM == kPair ? half : FORM == kWide ? quarter * 2 + half : (quarter & 1) * 2 + half;
+  part = FORM == kPair ? quarter : FORM == kWide ? 0 : (quarter < 2 ? 0 : 1);
+}
+
 // Final accumulator of work item `it` (S in tensor-memory columns at `sc`,
 // plus the running sum at `rc` unless `first`), columns [cbeg, cbeg + ncol):
 // the group of G warps holding one block of 32 filters' parts (this warp's
@@ -235,16 +280,17 @@ __device__ __forceinline__ void convert_kgroups(const float *src, size_t plane, 
 // share of the filters (a half, or a quarter) and stores them, so no warp
 // waits on another's stores.  `release` (or null): arrived on once this
 // warp's last accumulator load is done.
-template <int TERMS, bool PAIR>
+template <int TERMS, int FORM>
 __device__ __forceinline__ void store_tile_columns(const BankParams &p, const Item &it, uint32_t sc, uint32_t rc,
                                                    bool first, int cbeg, int ncol, float *tiles, int bar_id,
                                                    int quarter, int part, int lane, uint64_t *release) {
   const ConvGeom &g = p.g;
-  constexpr int G = PAIR ? 4 : 2;  // parts (warps) per group
-  const int bar_count = 32 * G;
+  constexpr int G = form_parts(FORM);  // parts (warps) per group
+  // tap b's rows: their sums sit one position to the right
+  const bool shifted = FORM == kPair ? (quarter & 1) != 0 : FORM == kWidePair ? quarter >= 2 : false;
   const bool relu = (g.flags & CCT_FLAG_RELU) != 0;
   const size_t opl = (size_t)g.OH * g.OW;
-  const int limit = PAIR ? p.tile_adv : p.N;  // columns of the tile with complete sums
+  const int limit = pairs_taps(FORM) ? p.tile_adv : p.N;  // columns of the tile with complete sums
   const int p0 = it.tile * p.tile_adv;
   // grid position (Y, X) of band `band` -> output (up*Y + rho, up*(band*BW + X) + kap)
   const int rho = it.ph / p.up, kap = it.ph - rho * p.up;
@@ -252,7 +298,7 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
   const int bw = min(p.BW, (g.OW - kap + p.up - 1) / p.up - it.band * p.BW);     // valid columns of the band
   const size_t ors = (size_t)p.up * g.OW;                                          // output row stride of a grid row
   // the group's 32 filters
-  const int fb = it.nb * p.fblock + (PAIR ? 0 : (quarter & 1) * 32);
+  const int fb = it.nb * p.fblock + (FORM == kPair ? 0 : FORM == kWide ? quarter * 32 : (quarter & 1) * 32);
   float *ybase0 = p.y + (size_t)it.b * g.groups * opl + (size_t)rho * g.OW + (size_t)it.band * p.BW * p.up + kap +
                   (size_t)fb * opl;
   // The next chunk's accumulator load is in flight while a chunk is combined
@@ -261,15 +307,15 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
   uint32_t n16[16], ne = 0;
   auto issue = [&](int c) {
     tmem_ld16(sc + c, n16);
-    // paired taps: tap b's rows (quarters 1, 3) also need column c + 16
-    if (PAIR && (quarter & 1) && c + 16 < p.N) tmem_ld1(sc + c + 16, ne);
+    // paired taps: tap b's rows also need column c + 16
+    if (shifted && c + 16 < p.N) tmem_ld1(sc + c + 16, ne);
   };
-  constexpr bool kAhead = TERMS == 2 && !PAIR;
+  constexpr bool kAhead = TERMS == 2 && FORM == kPlain;
   if (kAhead) issue(cbeg);
   for (int c = cbeg; c < cbeg + ncol; c += 16) {
     if (!kAhead) issue(c);
     tc_wait_ld();
-    const bool ext = PAIR && (quarter & 1) && c + 16 < p.N;
+    const bool ext = shifted && c + 16 < p.N;
     uint32_t s16[16], r16[16], e1 = ne, e2 = 0;
 #pragma unroll
     for (int t = 0; t < 16; ++t) s16[t] = n16[t];
@@ -282,6 +328,14 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
 #pragma unroll
     for (int t = 0; t < 16; ++t) v[t] = __uint_as_float(s16[t]) + (first ? 0.0f : __uint_as_float(r16[t]));
     v[16] = ext ? __uint_as_float(e1) + (first ? 0.0f : __uint_as_float(e2)) : 0.0f;
+    if (wide_form(FORM)) {  // the small sums, in columns of their own
+      tmem_ld16(sc + kAccCols / 2 + c, s16);
+      if (ext) tmem_ld1(sc + kAccCols / 2 + c + 16, e1);
+      tc_wait_ld();
+#pragma unroll
+      for (int t = 0; t < 16; ++t) v[t] += __uint_as_float(s16[t]);
+      if (ext) v[16] += __uint_as_float(e1);
+    }
     if (release && c + 16 >= cbeg + ncol) {  // the accumulator is read: release it
       tc_fence_before();
       __syncwarp();
@@ -289,12 +343,11 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
     }
     {
       float *mine = tiles + part * kXchFloats + lane * kXchPitch;
-      const bool sh = PAIR && (quarter & 1);  // tap b's sums sit one position to the right
 #pragma unroll
-      for (int t = 0; t < 16; ++t) mine[t] = sh ? v[t + 1] : v[t];
+      for (int t = 0; t < 16; ++t) mine[t] = shifted ? v[t + 1] : v[t];
     }
     if (kAhead && c + 16 < cbeg + ncol) issue(c + 16);
-    named_sync(bar_id, bar_count);  // every part of the chunk is in place
+    group_sync<G>(bar_id);  // every part of the chunk is in place
     // this warp's share: the parts of its filters, all loaded before the
     // barrier that lets the group overwrite the tiles
     float w[16];
@@ -320,7 +373,7 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
         for (int q = 0; q < G; ++q)
           w[k * G + q] = tiles[q * kXchFloats + (2 * (part * (16 / G) + k) + fl) * kXchPitch + t0];
     }
-    named_sync(bar_id, bar_count);  // the tiles may be rewritten
+    group_sync<G>(bar_id);  // the tiles may be rewritten
     const int Gp = p0 + c + t0;
     const int Y = Gp / p.P, X = Gp - Y * p.P;
     const bool ok = Y < ohv && X < bw && c + t0 < limit;
@@ -364,7 +417,7 @@ __device__ __forceinline__ bool helpers_store_last(const BankParams &p) { return
 
 // CB16: 16-plane blocks (the converters pair their (phase, position) items);
 // a separate instance, so the other plane blocks' code is unchanged.
-template <int TERMS, bool PAIR, bool CB16>
+template <int TERMS, int FORM, bool CB16>
 __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_constant__ BankParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ Bars bars;
@@ -493,28 +546,28 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
       // accumulator (one segment per item, so the phases of each buffer are
       // waited in order), then store through tiles in the halo, which no MMA
       // reads any more.
-      constexpr int G = PAIR ? 4 : 2;
+      constexpr int G = form_parts(FORM);
       int i_last = blockIdx.x, nitems = 0;
       for (int i = blockIdx.x; i < p.total; i += gridDim.x, ++nitems) i_last = i;
       const uint32_t u = (uint32_t)nitems - 1;  // the last item's segment (one per item)
       const int bi = (int)(u & 1);
       const uint32_t use = u >> 1;
       const int quarter = warp & 3, chalf = warp >> 2;  // converter warps 0-7: lane quarter, column quarter
-      const int grp = PAIR ? chalf : (quarter & 1) * 2 + chalf;
-      const int part = PAIR ? quarter : (quarter < 2 ? 0 : 1);
-      const int bar_id = 6 + grp;  // epilogue groups use 2-5
+      int grp, part;
+      group_of<FORM>(quarter, chalf, grp, part);
+      const int bar_id = 6 + grp;  // epilogue groups use 2-5 (groups of one warp none)
       // every converter warp comes here, failed or not, so both (or all
       // four) warps of a group reach the barrier; they agree to skip if any
       // of them failed or the wait gives up
       bool bad = failed || *abort_flag != 0;
       if (!bad) bad = !mbar_wait(&bars.dfull[bi], use & 1, p.err);
-      bad = named_sync_or(bar_id, 32 * G, bad);
+      bad = group_sync_or<G>(bar_id, bad);
       if (!bad) {
         tc_fence_after();
         const uint32_t sc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)bi * kAccCols;
         float *tiles = reinterpret_cast<float *>(halo) + grp * G * kXchFloats;
         const int ncol = p.N / 4;
-        store_tile_columns<TERMS, PAIR>(p, decode(p, i_last), sc, sc, true, p.N / 2 + chalf * ncol, ncol, tiles,
+        store_tile_columns<TERMS, FORM>(p, decode(p, i_last), sc, sc, true, p.N / 2 + chalf * ncol, ncol, tiles,
                                         bar_id, quarter, part, lane, nullptr);
       } else {
         *abort_flag = 1;
@@ -522,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer
-    using ML = MmaList<TERMS, PAIR>;
+    using ML = MmaList<TERMS, wide_form(FORM)>;
     const uint32_t idesc = idesc_bf16_f32(128, p.N);
     // Operand descriptors are a template (layout, strides) plus the address
     // in 16-byte units; shared-memory addresses stay below 256 KB, so the
@@ -552,14 +605,14 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
     int table_key = -1;    // (sub-filter width, units) the unit table holds
     bool failed = false;
     for (int i = blockIdx.x; i < p.total && !failed; i += gridDim.x) {
-      const ItemUnits iu = item_units<PAIR>(p, decode(p, i));
+      const ItemUnits iu = item_units<FORM>(p, decode(p, i));
       if (iu.ts * 1024 + iu.nu != table_key) {
         // (re)written whenever the sub-filter width or the unit count changes
         // (output phases of UpsampleInput), so every unit k < nu has its entry
         // B offset of each unit (paired: of its first tap), in 16-byte units
-        const int hs = PAIR ? (iu.ts + 1) / 2 : iu.ts;  // units per filter row
+        const int hs = pairs_taps(FORM) ? (iu.ts + 1) / 2 : iu.ts;  // units per filter row
         for (int k = lane; k < iu.nu; k += 32) {
-          const int tap = (k / hs) * p.tstride + (PAIR ? 2 : 1) * (k % hs);
+          const int tap = (k / hs) * p.tstride + (pairs_taps(FORM) ? 2 : 1) * (k % hs);
           unit_boff[k] = (uint32_t)p.tap_phase[tap] * TERMS * part16 + (uint32_t)p.tap_off[tap];
         }
         __syncwarp();
@@ -567,7 +620,10 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
       }
       const int tstages = p.NCB * iu.nst;
       int seg_left = 0, done = 0, bi = 0;
-      bool first = false;
+      // first: the next MMA starts a segment's (big) sum; first_small, wide forms:
+      // it starts the small sums, which stay in their columns for the whole item
+      // (a 2^-8 part of the result: their accumulation needs no promotion)
+      bool first = false, first_small = true;
       for (int cb = 0; cb < p.NCB && !failed; ++cb, ++hb) {
         const int buf = hb & 1;
         failed = __any_sync(0xffffffffu, *abort_flag || !mbar_wait(&bars.hfull[buf], (hb >> 1) & 1, p.err));
@@ -597,11 +653,12 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
               for (int j = 0; j < p.KS; ++j) {
 #pragma unroll
                 for (int m = 0; m < ML::n; ++m) {
-                  mma_bf16_ss(dt, desc_word(a_hi, alo + aoff[m] + 16u * j),
+                  const bool small = wide_form(FORM) && m > 0;
+                  mma_bf16_ss(dt + (small ? kAccCols / 2 : 0u), desc_word(a_hi, alo + aoff[m] + 16u * j),
                               desc_word(b_hi, blo + boff[m] + (uint32_t)j * kstep_b16), idesc,
-                              (first && m == 0) ? 0u : 1u);
-                  first = false;
+                              (m == 0 && first) || (m == 1 && wide_form(FORM) && first_small) ? 0u : 1u);
                 }
+                first = first_small = false;
               }
             }
             tc_commit(&bars.empty[s]);  // the stage may be refilled once these MMAs are done
@@ -611,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
             s = 0;
             sph ^= 1u;
           }
-          first = false;
+          first = first_small = false;
           ++done;
           if (--seg_left == 0) {
             if (elect_one()) tc_commit(&bars.dfull[bi]);
@@ -641,7 +698,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
       uint32_t sph = 0;   // parity of the slot's current fill
       bool ok = true;
       for (int i = blockIdx.x; ok && i < p.total && !*abort_flag; i += gridDim.x) {
-        const ItemUnits iu = item_units<PAIR>(p, decode(p, i));
+        const ItemUnits iu = item_units<FORM>(p, decode(p, i));
         const int NU = iu.nu;
         const uint8_t *src = p.bpack + iu.chunk0 * p.chunk_bytes;
         for (int cb = 0; ok && cb < p.NCB; ++cb)
@@ -675,13 +732,13 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
     // corrections, tap b's one grid position to the right.  The warps holding
     // the parts of one block of 32 filters for the same columns form a group
     // (two warps, or with paired taps four): store_tile_columns.
-    constexpr int G = PAIR ? 4 : 2;  // parts (warps) per group
+    constexpr int G = form_parts(FORM);   // parts (warps) per group
     const int ew = warp - kEpiWarp0;
     const int quarter = warp & 3;         // tensor-memory lanes this warp may access
     const int half = ew >> 2;             // column half
-    const int grp = PAIR ? half : (quarter & 1) * 2 + half;
-    const int part = PAIR ? quarter : (quarter < 2 ? 0 : 1);  // this warp's part, and its share of filters
-    const int bar_id = 2 + grp, bar_count = 32 * G;
+    int grp, part;                        // this warp's part, and its share of filters
+    group_of<FORM>(quarter, half, grp, part);
+    const int bar_id = 2 + grp;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     float *tiles = xch + grp * G * kXchFloats;  // the group's part tiles, [part][filter][pitch 17]
     const bool helped = helpers_store_last(p);
@@ -689,7 +746,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
     bool failed = false;
     for (int i = blockIdx.x; i < p.total && !failed; i += gridDim.x) {
       const Item it = decode(p, i);
-      const ItemUnits iu = item_units<PAIR>(p, it);
+      const ItemUnits iu = item_units<FORM>(p, it);
       const int nseg = (p.NCB * iu.nst + p.seg_stages - 1) / p.seg_stages;  // accumulation segments
       // the CTA's last tile: the converters store the upper half of the columns
       const bool last_item = i + (int)gridDim.x >= p.total;
@@ -699,7 +756,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
         const int bi = p.promote ? 0 : (int)(u & 1);
         const uint32_t use = p.promote ? u : (u >> 1);
         bool bad = *abort_flag != 0 || !mbar_wait(&bars.dfull[bi], use & 1, p.err);
-        bad = named_sync_or(bar_id, bar_count, bad);  // the group agrees
+        bad = group_sync_or<G>(bar_id, bad);  // the group agrees
         if (bad) {
           failed = true;
           break;
@@ -728,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
           continue;
         }
         // last segment: out = S (+ R) for every part of each filter
-        store_tile_columns<TERMS, PAIR>(p, it, sc, rc, first, cbeg, ncol, tiles, bar_id, quarter, part, lane,
+        store_tile_columns<TERMS, FORM>(p, it, sc, rc, first, cbeg, ncol, tiles, bar_id, quarter, part, lane,
                                         &bars.dempty[bi]);
       }
     }
@@ -744,32 +801,35 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
 
 // Pack the filter bank into per-chunk operand images: chunk (output phase,
 // nb, cb, unit) = arows x CB bf16, column ci = plane cb*CB + ci, the filter
-// value of the tap (flipped for convolution).  A unit is one tap, with row
-// blocks of 64 as block_term() lists and row n of a block = filter nb*64 + n;
-// or, paired, two taps a, a + 1 of a filter row, with row blocks of 32 as
-// pair_block_term() and pair_block_tap() list and row n of a block = filter
-// nb*32 + n (tap a + 1 past the row's end is 0).  With UpsampleInput the
-// taps of a unit are those of its phase's sub-filter.  Layout: core matrices
-// of 8 rows x 8 columns (128 bytes), row groups SBO = CB*16 bytes apart,
-// column groups LBO = 128 bytes apart.  Rows or columns past the real counts
-// are 0.
+// value of the tap (flipped for convolution).  A chunk is blocks of SR source
+// rows (64, wide forms 128), each the rows' values in one split term, or zero,
+// as block_term() lists them (wide: the terms in order).  A source row is a
+// filter nb*fblock + n of the unit's tap, or, in the pairing forms, the first
+// half of the rows are tap a of the unit's filters and the second half tap a + 1
+// (0 past the filter row's end).  With UpsampleInput the taps of a unit are those
+// of its phase's sub-filter.  Layout: core matrices of 8 rows x 8 columns (128
+// bytes), row groups SBO = CB*16 bytes apart, column groups LBO = 128 bytes
+// apart.  Rows or columns past the real counts are 0.
 //
-// One thread per core-matrix row (8 planes of one filter row: 8 loads in
-// flight, one 16-byte store).  The launch is one CTA of 128 threads per SM:
-// at 32 registers a thread its four warps fit in the registers a
-// filter-bank CTA leaves free on each SM sub-partition, so with programmatic
-// serialisation it is resident before the previous launch ends and runs the
-// moment that launch is done (measured: 1.6 / 2.3 us less per forward /
-// backward launch than one thread per value in 256-thread CTAs).
-template <bool PAIR>
+// One thread per 8 planes of one source row: 8 loads in flight, then one
+// 16-byte store for each block (loading the values again for every block, from
+// one CTA per SM, took 147 us for a 3x3 512 -> 512 bank; 20 us now).  The
+// launch is one CTA of 128 threads per SM: at 32 registers a thread its four
+// warps fit in the registers a filter-bank CTA leaves free on each SM
+// sub-partition, so with programmatic serialisation it is resident before the
+// previous launch ends and runs the moment that launch is done (measured: 1.6 /
+// 2.3 us less per forward / backward launch than one thread per value in
+// 256-thread CTAs).
+template <int FORM>
 __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __grid_constant__ BankParams p,
                                                                      const float *__restrict__ f,
                                                                      uint8_t *__restrict__ out) {
+  constexpr int SR = wide_form(FORM) ? 128 : 64;
   const ConvGeom &g = p.g;
-  const int CB8 = p.CB / 8, arows = p.arows;
+  const int CB8 = p.CB / 8, nblk = p.arows / SR;
   // every (phase, block, plane block, unit) slot of the largest phase; the
   // units a phase lacks are skipped.  Below 2^31 (checked at launch).
-  const int total = p.nph_out * p.nblocks * p.NCB * p.nunits * arows * CB8;
+  const int total = p.nph_out * p.nblocks * p.NCB * p.nunits * SR * CB8;
   // the previous kernel (the last launch that read the packed operand) must
   // be done before it is rewritten; the consuming kernel may be scheduled now
   grid_dependency_wait();
@@ -777,8 +837,8 @@ __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __gri
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
     const int c8 = idx % CB8;
     int rest = idx / CB8;
-    const int row = rest % arows;
-    rest /= arows;
+    const int row = rest % SR;
+    rest /= SR;
     const int unit = rest % p.nunits;
     rest /= p.nunits;
     const int cb = rest % p.NCB;
@@ -787,20 +847,11 @@ __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __gri
     Item it{};
     it.ph = rest / p.nblocks;
     it.nb = nb;
-    const ItemUnits iu = item_units<PAIR>(p, it);
+    const ItemUnits iu = item_units<FORM>(p, it);
     if (unit >= iu.nu) continue;
-    const int hs = PAIR ? (iu.ts + 1) / 2 : iu.ts;
-    int part, k, ss;
-    if (PAIR) {
-      const int blk = row >> 5;
-      part = pair_block_term(blk);
-      k = nb * 32 + (row & 31);
-      ss = 2 * (unit % hs) + pair_block_tap(blk);
-    } else {
-      part = block_term(p.terms, row >> 6);
-      k = nb * 64 + (row & 63);
-      ss = unit % hs;
-    }
+    const int hs = pairs_taps(FORM) ? (iu.ts + 1) / 2 : iu.ts;
+    const int k = nb * p.fblock + (pairs_taps(FORM) ? row % (SR / 2) : row);
+    const int ss = pairs_taps(FORM) ? 2 * (unit % hs) + row / (SR / 2) : unit % hs;
     const int rr = unit / hs;
     int r = rr, s = ss;
     if (p.up > 1) {
@@ -808,7 +859,7 @@ __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __gri
       r = p.up_r0[rho] + p.up * rr;
       s = p.up_s0[it.ph - rho * p.up] + p.up * ss;
     }
-    const bool live = part >= 0 && ss < iu.ts && r < g.R && s < g.S && k < g.groups;
+    const bool live = ss < iu.ts && r < g.R && s < g.S && k < g.groups;
     const int src = g.orient == CCT_CONVOLUTION ? (g.R - 1 - r) * g.S + (g.S - 1 - s) : r * g.S + s;
     // filter plane of (filter k, plane c), as plane_pair gives it: k*n + c
     // for projectFrame, c*groups + k for backProjectFrame
@@ -820,44 +871,50 @@ __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __gri
     float a[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) a[e] = (live && c0 + e < g.n) ? __ldg(fp + (size_t)e * fstride) : 0.0f;
-    uint32_t w[4];
-#pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      float v[2];
-#pragma unroll
-      for (int d = 0; d < 2; ++d) {
-        const float x = a[e + d];
-        const float h = __bfloat162float(__float2bfloat16_rn(x));
-        if (part <= 0) {
-          v[d] = h;  // a zero block holds x = 0
-        } else if (p.terms == 2) {
-          v[d] = x - h;  // rounded to bf16 below
-        } else {
-          const float m = __bfloat162float(__float2bfloat16_rn(x - h));
-          v[d] = part == 1 ? m : (x - h) - m;
-        }
-      }
-      const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[0], v[1]);  // v[0] in the low half
-      w[e / 2] = *reinterpret_cast<const uint32_t *>(&b2);
-    }
     const size_t chunk = iu.chunk0 + (size_t)cb * iu.nu + unit;
-    const uint32_t off = (uint32_t)((row >> 3) * (p.CB * 16) + c8 * 128 + (row & 7) * 16);
-    *reinterpret_cast<uint4 *>(out + chunk * ((size_t)arows * p.CB * 2) + off) = make_uint4(w[0], w[1], w[2], w[3]);
+    uint8_t *dst = out + chunk * ((size_t)p.arows * p.CB * 2) +
+                   (uint32_t)((row >> 3) * (p.CB * 16) + c8 * 128 + (row & 7) * 16);
+    for (int b = 0; b < nblk; ++b, dst += (size_t)SR * p.CB * 2) {
+      const int term = wide_form(FORM) ? b : block_term(p.terms, b);
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        float v[2];
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          const float x = a[e + d];
+          const float h = __bfloat162float(__float2bfloat16_rn(x));
+          if (term < 0) {
+            v[d] = 0.0f;
+          } else if (term == 0) {
+            v[d] = h;
+          } else if (p.terms == 2) {
+            v[d] = x - h;  // rounded to bf16 below
+          } else {
+            const float m = __bfloat162float(__float2bfloat16_rn(x - h));
+            v[d] = term == 1 ? m : (x - h) - m;
+          }
+        }
+        const __nv_bfloat162 b2 = __floats2bfloat162_rn(v[0], v[1]);  // v[0] in the low half
+        w[e / 2] = *reinterpret_cast<const uint32_t *>(&b2);
+      }
+      *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
   }
 }
 
 std::mutex g_bank_mu;
 std::unordered_map<uint64_t, size_t> g_bank_attr;
 
-template <int TERMS, bool PAIR, bool CB16>
+template <int TERMS, int FORM, bool CB16>
 int launch_terms(const BankParams &p, cudaStream_t st) {
-  auto kern = bank_tc_kernel<TERMS, PAIR, CB16>;
+  auto kern = bank_tc_kernel<TERMS, FORM, CB16>;
   {
     // Dynamic shared memory above 48 KB needs the opt-in attribute; keep the
     // largest size set so far per (device, instance).
     int dev = 0;
     cudaGetDevice(&dev);
-    const uint64_t key = ((uint64_t)dev << 32) | (uint64_t)(TERMS * 4 + (PAIR ? 2 : 0) + (CB16 ? 1 : 0));
+    const uint64_t key = ((uint64_t)dev << 32) | (uint64_t)(TERMS * 8 + FORM * 2 + (CB16 ? 1 : 0));
     std::lock_guard<std::mutex> lk(g_bank_mu);
     size_t &have = g_bank_attr[key];
     if (have < p.smem_bytes) {
@@ -879,7 +936,11 @@ int pos_mod(int a, int b) { return ((a % b) + b) % b; }
 
 }  // namespace
 
-bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
+namespace {
+
+// The plan of one form, or false where the form or the kernel does not take the
+// shape.  *cost: modelled MMA cycles of the longest-running CTA.
+bool plan_form(const ConvGeom &g, int terms, int form, int sms, BankParams *out, double *cost_out) {
   if (g.mode != CCT_PROJECT_FRAME_BLOCK_REDUCE_SUM && g.mode != CCT_BACK_PROJECT_FRAME_BLOCK_REDUCE_SUM)
     return false;
   if (terms != 2 && terms != 3) return false;
@@ -931,11 +992,13 @@ bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
     sq_max = g.S;
   }
   if (rq_max * p.tstride > kBankMaxTaps) return false;
-  // Banks of at most 32 filters would leave half of each 128-row MMA empty:
-  // two taps of a filter row share it instead (stride-1 grids only, where
-  // tap a + 1 reads one grid position past tap a).
-  p.pair = (terms == 2 && g.groups <= 32 && d == 1 && sq_max >= 2) ? 1 : 0;
-  p.fblock = p.pair ? 32 : 64;
+  // paired taps: stride-1 grids only, where tap a + 1 reads one grid position
+  // past tap a
+  p.form = form;
+  p.pair = pairs_taps(form) ? 1 : 0;
+  if (p.pair && (d != 1 || sq_max < 2)) return false;
+  if (form == kPair && (terms != 2 || g.groups > 32)) return false;
+  p.fblock = form == kPair ? 32 : form == kWide ? 128 : 64;
   p.nblocks = (g.groups + p.fblock - 1) / p.fblock;
   // units per phase: sub-filter rows x (columns, or column pairs)
   auto units_of = [&](int rows, int cols) { return rows * (p.pair ? (cols + 1) / 2 : cols); };
@@ -944,8 +1007,9 @@ bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
     const int nu = u > 1 ? units_of(p.up_rq[ph / u], p.up_sq[ph % u]) : units_of(g.R, g.S);
     p.nunits = std::max(p.nunits, nu);
   }
-  p.nmma = terms == 2 ? 2 : 5;
-  p.arows = terms == 2 ? 192 : 448;
+  const bool wide = wide_form(form);
+  p.nmma = wide ? (terms == 2 ? 3 : 6) : (terms == 2 ? 2 : 5);
+  p.arows = wide ? 128 * terms : (terms == 2 ? 192 : 448);
   const size_t xch_bytes = kXchBytes;
   const int NU = p.nunits;
   int phase_of[2][2] = {{-1, -1}, {-1, -1}};
@@ -986,6 +1050,7 @@ bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
     const int P = BW + dc;
     const long long npos = (long long)p.OHq * P;
     for (int N : {256, 224, 192, 160, 128, 96, 64}) {
+      if (wide && N > 128) continue;  // big and small sums share the accumulator's columns
       const int adv = p.pair ? N - 4 : N;  // paired: the last 4 positions of a tile lack tap b's sums
       const long long tiles = (npos + adv - 1) / adv;
       const int L = ((N + dr * P + dc) + 7) & ~7;
@@ -1081,18 +1146,50 @@ bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
   }
   p.pack_bytes = chunks * p.chunk_bytes;
   *out = p;
+  *cost_out = best_cost * p.NCB * p.KS * NU * p.nmma;
+  return true;
+}
+
+}  // namespace
+
+bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
+  // Banks of at most 32 filters would leave half of each 128-row MMA empty: two
+  // taps of a filter row share it instead where they can.
+  BankParams p{}, w{};
+  double cost = 0.0, wcost = 0.0;
+  const bool paired = terms == 2 && plan_form(g, terms, kPair, sms, &p, &cost);
+  const bool ok = paired || plan_form(g, terms, kPlain, sms, &p, &cost);
+  if (!ok) return false;
+  p.pack_limit = p.pack_bytes;
+  // The wide forms where the model says they take fewer MMA cycles: 128 filters
+  // (from 0.95: 256 -> 512 planes on 8x 28x28, three terms 134 -> 94 us, two terms
+  // 70 -> 62), or 64 filters x two taps, whose smaller tiles convert and store more
+  // per position (from 0.78: three terms, 5x5 64 -> 32 planes on 16x 64x64, 0.74,
+  // 96 -> 85 us; 3x3 64 -> 64 on 8x 112x112, 0.83, 60 / 69 us).  Never a larger
+  // packed operand: whoever holds a fixed scratch for it keeps what it takes.
+  const int form = paired ? -1 : g.groups > 64 ? kWide : kWidePair;
+  if (form >= 0 && plan_form(g, terms, form, sms, &w, &wcost) && wcost < (form == kWide ? 0.95 : 0.78) * cost &&
+      w.pack_bytes <= p.pack_bytes) {
+    w.pack_limit = p.pack_bytes;
+    p = w;
+  }
+  *out = p;
   return true;
 }
 
 int launch_bank_pack(const BankParams &p, const float *f, uint8_t *packed, cudaStream_t st) {
-  const long long total = (long long)p.nph_out * p.nblocks * p.NCB * p.nunits * p.arows * (p.CB / 8);
+  const long long total = (long long)p.nph_out * p.nblocks * p.NCB * p.nunits * (wide_form(p.form) ? 128 : 64) * (p.CB / 8);
   if (total > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "packed filter operand too large");
-  // one CTA per SM (more would wait for the filter-bank CTAs to leave)
-  const int blocks = (int)std::min<long long>((total + kPackThreads - 1) / kPackThreads, p.sms);
-  const int rc = p.pair ? launch_pdl(bank_pack_kernel<true>, dim3(blocks), dim3(kPackThreads), 0, st,
-                                     "bank_pack_kernel launch", p, f, packed)
-                        : launch_pdl(bank_pack_kernel<false>, dim3(blocks), dim3(kPackThreads), 0, st,
-                                     "bank_pack_kernel launch", p, f, packed);
+  // One CTA per SM (more would wait for the filter-bank CTAs to leave) while a
+  // thread then packs one row; a larger bank takes up to 16 (3x3 256 -> 256 planes on
+  // 8x 28x28, dynamic filter: 75 us with one, 66 with more).
+  const long long ctas = (total + kPackThreads - 1) / kPackThreads;
+  const int blocks = (int)std::min<long long>(ctas, ctas > 1LL * p.sms ? 16LL * p.sms : p.sms);
+  const auto kern = p.form == kPair       ? bank_pack_kernel<kPair>
+                    : p.form == kWide     ? bank_pack_kernel<kWide>
+                    : p.form == kWidePair ? bank_pack_kernel<kWidePair>
+                                          : bank_pack_kernel<kPlain>;
+  const int rc = launch_pdl(kern, dim3(blocks), dim3(kPackThreads), 0, st, "bank_pack_kernel launch", p, f, packed);
   if (rc) return rc;
   count_launches(1);
   return check_cuda(cudaGetLastError(), "bank_pack_kernel launch");
@@ -1108,9 +1205,12 @@ int launch_bank_tc(const BankParams &p, const float *x, float *y, const uint8_t 
   q.bpack = packed;
   q.err = err;
   const bool cb16 = p.CB == 16;
-  if (p.pair) return cb16 ? launch_terms<2, true, true>(q, st) : launch_terms<2, true, false>(q, st);
-  if (p.terms == 2) return cb16 ? launch_terms<2, false, true>(q, st) : launch_terms<2, false, false>(q, st);
-  return cb16 ? launch_terms<3, false, true>(q, st) : launch_terms<3, false, false>(q, st);
+#define CCT_BANK_CASE(TT, FF) \
+  if (p.terms == TT && p.form == FF) return cb16 ? launch_terms<TT, FF, true>(q, st) : launch_terms<TT, FF, false>(q, st);
+  CCT_BANK_CASE(2, kPlain) CCT_BANK_CASE(2, kPair) CCT_BANK_CASE(2, kWide) CCT_BANK_CASE(2, kWidePair)
+  CCT_BANK_CASE(3, kPlain) CCT_BANK_CASE(3, kWide) CCT_BANK_CASE(3, kWidePair)
+#undef CCT_BANK_CASE
+  return set_error(CCT_ENOTSUP, "filter-bank kernel: no form %d of %d terms", p.form, p.terms);
 }
 
 }  // namespace cct
@@ -1121,7 +1221,7 @@ bool frame_tc_choose(const ConvGeom &g, int precision, int sms, FrameTcChoice *o
   FrameTcChoice c{};
   BankParams bp{};
   const bool bank_ok = bank_tc_plan(g, precision == CCT_PREC_BF16X6 ? 3 : 2, sms, &bp);
-  if (bank_ok && (bp.pair || g.groups > 32 || precision != CCT_PREC_BF16X3)) {
+  if (bank_ok && (bp.form == kPair || g.groups > 32 || precision != CCT_PREC_BF16X3)) {
     c.bank = true;
     c.bp = bp;
     c.pack_bytes = bp.pack_bytes;

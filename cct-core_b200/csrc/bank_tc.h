@@ -14,13 +14,14 @@ constexpr int kBankMaxUp = 4;       // UpsampleInput steps the kernel takes
 struct BankParams {
   ConvGeom g;
   int terms;        // bf16 terms per split value: 2 (BF16X3) or 3 (BF16X6)
-  int pair;         // 1: banks of at most 32 filters, two taps of a filter row per MMA
-  int fblock;       // filters per block: 64, or 32 when paired
+  int form;         // how a block's filters, taps and sums fill the MMAs (bank_tc.cu)
+  int pair;         // 1: two taps of a filter row per MMA
+  int fblock;       // filters per block: 32, 64 or 128
   int nunits;       // reduction units per plane block: taps, or tap pairs (R * ceil(S/2));
                     // with UpsampleInput the largest over the output phases
   int tile_adv;     // positions a tile advances: N, or N - 4 when paired
-  int nmma;         // MMAs per 16-deep k-step: 2 or 5
-  int arows;        // rows of one packed filter chunk (64 per block: 192 or 448)
+  int nmma;         // MMAs per 16-deep k-step: 2 or 5 (wide forms: 3 or 6)
+  int arows;        // rows of one packed filter chunk: 192 or 448 (wide: 256 or 384)
   int CB;           // input planes per halo block (multiple of 16)
   int NCB;          // ceil(n / CB)
   int KS;           // 16-deep k-steps per chunk: CB / 16
@@ -62,6 +63,7 @@ struct BankParams {
   int sms;               // SMs of the device
   size_t smem_bytes;     // dynamic shared memory
   size_t pack_bytes;     // bytes of the packed filter operand
+  size_t pack_limit;     // the same in the narrow form: what a fixed scratch is compared with
   int after_pack;        // 1: the preceding grid in the stream is this launch's filter pack
   const float *x;
   const uint8_t *bpack;

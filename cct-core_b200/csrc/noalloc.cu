@@ -87,11 +87,13 @@ extern "C" int cct_conv_run_noalloc(const cct_conv_desc *desc, const float *imag
   FrameTcChoice tc;  // the same kernel and tile plan a plan for this descriptor runs
   if (!frame_tc_choose(g, CCT_PREC_BF16X3, sms, &tc))
     return set_error(CCT_ENOTSUP, "shape outside the tensor-core frame kernels (sampling or tile size)");
-  if (tc.pack_bytes > kNoAllocScratchBytes)
+  // the limit is on the narrow forms' operand, which the wide forms' never exceeds
+  const size_t need = tc.bank ? tc.bp.pack_limit : tc.pack_bytes;
+  if (need > kNoAllocScratchBytes)
     return set_error(CCT_EINVAL,
                      "packed filter operand needs %zu bytes; the allocation-free entry point holds "
                      "at most %zu",
-                     tc.pack_bytes, kNoAllocScratchBytes);
+                     need, kNoAllocScratchBytes);
 
   uint8_t *scratch = nullptr;
   rc = scratch_address(dev, &scratch);
