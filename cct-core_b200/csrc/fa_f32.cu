@@ -267,19 +267,39 @@ __global__ void __launch_bounds__(NW * 32)
 #pragma unroll
       for (int e = 0; e < NV; ++e) put(e, xp[e]);
       const int quads = Wg / 4, rest = Wg - 4 * quads;
-      for (int q = 0; q <= quads; q += NV) {
+      // a quad's gradients, and the image values it brings in, are read while the
+      // quad before it is multiplied
+      float4 gq[4];
 #pragma unroll
-        for (int u = 0; u < NV; ++u) {
-          if (q + u < quads) {
+      for (int jj = 0; jj < 4; ++jj) gq[jj] = gp[jj];
+      auto quad = [&](int q, int u) {
+        const float4 nx = xp[q + NV];
+        float4 gn[4];
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) tap(4 * u + jj, gp[4 * (q + u) + jj]);
-            put(u, xp[q + u + NV]);
-          } else if (q + u == quads) {
+        for (int jj = 0; jj < 4; ++jj) gn[jj] = gp[4 * (q + 1) + jj];  // past the last column: not used
 #pragma unroll
-            for (int jj = 0; jj < 3; ++jj)
-              if (jj < rest) tap(4 * u + jj, gp[4 * quads + jj]);
-          }
-        }
+        for (int jj = 0; jj < 4; ++jj) tap(4 * u + jj, gq[jj]);
+        put(u, nx);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) gq[jj] = gn[jj];
+      };
+      auto tail = [&](int u) {
+#pragma unroll
+        for (int jj = 0; jj < 3; ++jj)
+          if (jj < rest) tap(4 * u + jj, gq[jj]);
+      };
+      int q = 0;
+#pragma unroll 1
+      for (; q + NV <= quads; q += NV) {
+#pragma unroll
+        for (int u = 0; u < NV; ++u) quad(q + u, u);
+      }
+#pragma unroll
+      for (int u = 0; u < NV; ++u) {
+        if (q + u < quads)
+          quad(q + u, u);
+        else if (q + u == quads)
+          tail(u);
       }
       float *out = sums + (size_t)warp * OUTS + lane;
 #pragma unroll
