@@ -205,8 +205,26 @@ __device__ __forceinline__ ItemUnits item_units(const BankParams &p, const Item 
     r.ts = p.g.S;
   }
   r.nu = rows * (pairs_taps(FORM) ? (r.ts + 1) / 2 : r.ts);
-  r.nst = (r.nu + p.T - 1) / p.T;
+  r.nst = p.hblocks > 1 ? p.nst : (r.nu + p.T - 1) / p.T;
   r.chunk0 = (size_t)p.up_choff[it.ph] + (size_t)it.nb * p.NCB * r.nu;
+  return r;
+}
+
+// One halo block: a plane block of every input phase with every unit, or
+// (hblocks > 1, DownsampleOutput(2)) of one phase with the units that read it.
+struct Block {
+  int cb, u0, u1;
+};
+__device__ __forceinline__ Block block_of(const BankParams &p, const ItemUnits &iu, int blk) {
+  Block r;
+  r.cb = blk / p.hblocks;
+  r.u0 = 0;
+  r.u1 = iu.nu;
+  if (p.hblocks > 1) {
+    const int ph = blk - r.cb * p.hblocks;
+    r.u0 = p.ph_u0[ph];
+    r.u1 = p.ph_u0[ph + 1];
+  }
   return r;
 }
 
@@ -475,7 +493,9 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
       const int row0 = p.up > 1 ? p.up_sr[rho] : p.sr_min;
       const int col0 = it.band * p.BW + (p.up > 1 ? p.up_sc[kap] : p.sc_min);
       const float *xb = p.x + (size_t)it.b * g.n * plane;
-      for (int cb = 0; cb < p.NCB; ++cb, ++hb) {
+      for (int blk = 0; blk < p.NCB * p.hblocks; ++blk, ++hb) {
+        const int cb = blk / p.hblocks;
+        const int ph0 = p.hblocks > 1 ? blk - cb * p.hblocks : 0, nph = p.hblocks > 1 ? 1 : p.nphase;  // its phases
         const int buf = hb & 1;
         if (*abort_flag || !mbar_wait(&bars.hempty[buf], ((hb >> 1) & 1) ^ 1, p.err)) {
           failed = true;
@@ -488,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
           // 16-plane blocks: the (phase, position) items two at a time, both
           // items' loads issued before either is converted, so a thread has
           // as many loads in flight as with a 32-plane position
-          const int total = p.nphase * p.L;
+          const int total = nph * p.L;
           for (int it = threadIdx.x; it < total; it += 2 * kConvThreads) {
             const float *src[2];
             bool in[2];
@@ -499,8 +519,8 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
               const int ph = item / p.L, q = item - ph * p.L;
               const int G = p0 + q;
               const int Y = G / p.P, X = G - Y * p.P;
-              const int iy = g.down * (Y + row0) + p.phase_r[ph];
-              const int ix = g.down * (col0 + X) + p.phase_c[ph];
+              const int iy = g.down * (Y + row0) + p.phase_r[ph0 + ph];
+              const int ix = g.down * (col0 + X) + p.phase_c[ph0 + ph];
               int ry, rx;
               in[e] = border_map(g, iy, ix, ry, rx);
               src[e] = in[e] ? xc + (size_t)ry * g.W + rx : xc;
@@ -513,13 +533,13 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
             if (it + kConvThreads < total) store_kgroups<TERMS, 2>(vb, dst[1], kgs, p.part_bytes);
           }
         } else {
-          for (int ph = 0; ph < p.nphase; ++ph) {
+          for (int ph = 0; ph < nph; ++ph) {
             uint8_t *hph = hbase + (size_t)ph * TERMS * p.part_bytes;
             for (int q = threadIdx.x; q < p.L; q += kConvThreads) {
               const int G = p0 + q;
               const int Y = G / p.P, X = G - Y * p.P;
-              const int iy = g.down * (Y + row0) + p.phase_r[ph];
-              const int ix = g.down * (col0 + X) + p.phase_c[ph];
+              const int iy = g.down * (Y + row0) + p.phase_r[ph0 + ph];
+              const int ix = g.down * (col0 + X) + p.phase_c[ph0 + ph];
               int ry, rx;
               const bool in = border_map(g, iy, ix, ry, rx);
               const float *src = in ? xc + (size_t)ry * g.W + rx : xc;
@@ -612,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
         // B offset of each unit (paired: of its first tap), in 16-byte units
         const int hs = pairs_taps(FORM) ? (iu.ts + 1) / 2 : iu.ts;  // units per filter row
         for (int k = lane; k < iu.nu; k += 32) {
-          const int tap = (k / hs) * p.tstride + (pairs_taps(FORM) ? 2 : 1) * (k % hs);
+          const int tap = p.hblocks > 1 ? p.unit_tap[k] : (k / hs) * p.tstride + (pairs_taps(FORM) ? 2 : 1) * (k % hs);
           unit_boff[k] = (uint32_t)p.tap_phase[tap] * TERMS * part16 + (uint32_t)p.tap_off[tap];
         }
         __syncwarp();
@@ -624,13 +644,14 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
       // it starts the small sums, which stay in their columns for the whole item
       // (a 2^-8 part of the result: their accumulation needs no promotion)
       bool first = false, first_small = true;
-      for (int cb = 0; cb < p.NCB && !failed; ++cb, ++hb) {
+      for (int blk = 0; blk < p.NCB * p.hblocks && !failed; ++blk, ++hb) {
+        const Block bk = block_of(p, iu, blk);
         const int buf = hb & 1;
         failed = __any_sync(0xffffffffu, *abort_flag || !mbar_wait(&bars.hfull[buf], (hb >> 1) & 1, p.err));
         if (failed) break;
         tc_fence_after();
         const uint32_t hlo = b_lo0 + (uint32_t)buf * (p.halo_bytes >> 4);
-        for (int st = 0; st < iu.nst; ++st) {
+        for (int u0 = bk.u0; u0 < bk.u1; u0 += p.T) {
           if (seg_left == 0) {
             // a new accumulation segment: wait until its accumulator is free
             bi = p.promote ? 0 : (int)(u & 1);
@@ -646,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
           tc_fence_after();
           if (elect_one()) {
             const uint32_t dt = tmem + (uint32_t)bi * kAccCols;
-            const int u0 = st * p.T, u1 = min(iu.nu, u0 + p.T);
+            const int u1 = min(bk.u1, u0 + p.T);
             uint32_t alo = a_lo0 + (uint32_t)s * stage16;
             for (int k = u0; k < u1; ++k, alo += chunk16) {
               const uint32_t blo = hlo + unit_boff[k];
@@ -699,24 +720,24 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
       bool ok = true;
       for (int i = blockIdx.x; ok && i < p.total && !*abort_flag; i += gridDim.x) {
         const ItemUnits iu = item_units<FORM>(p, decode(p, i));
-        const int NU = iu.nu;
         const uint8_t *src = p.bpack + iu.chunk0 * p.chunk_bytes;
-        for (int cb = 0; ok && cb < p.NCB; ++cb)
-          for (int st = 0; st < iu.nst; ++st, ++q) {
+        for (int blk = 0; ok && blk < p.NCB * p.hblocks; ++blk) {
+          const Block bk = block_of(p, iu, blk);
+          for (int u0 = bk.u0; u0 < bk.u1; u0 += p.T, ++q) {
             if (!mbar_wait(&bars.empty[s], sph ^ 1u, p.err)) {
               ok = false;
               break;
             }
-            const int t0 = st * p.T;
-            const uint32_t bytes = (uint32_t)min(p.T, NU - t0) * p.chunk_bytes;
+            const uint32_t bytes = (uint32_t)min(p.T, bk.u1 - u0) * p.chunk_bytes;
             mbar_arrive_expect_tx(&bars.full[s], bytes);
-            bulk_load(stage + (size_t)s * p.stage_bytes, src + ((size_t)cb * NU + t0) * p.chunk_bytes, bytes,
+            bulk_load(stage + (size_t)s * p.stage_bytes, src + ((size_t)bk.cb * iu.nu + u0) * p.chunk_bytes, bytes,
                       &bars.full[s]);
             if (++s == p.stages) {
               s = 0;
               sph ^= 1u;
             }
           }
+        }
       }
       if (!ok) *abort_flag = 1;
       if (*abort_flag) {
@@ -851,8 +872,9 @@ __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __gri
     if (unit >= iu.nu) continue;
     const int hs = pairs_taps(FORM) ? (iu.ts + 1) / 2 : iu.ts;
     const int k = nb * p.fblock + (pairs_taps(FORM) ? row % (SR / 2) : row);
-    const int ss = pairs_taps(FORM) ? 2 * (unit % hs) + row / (SR / 2) : unit % hs;
-    const int rr = unit / hs;
+    const int uo = p.hblocks > 1 ? p.unit_tap[unit] : unit;  // units in filter order
+    const int ss = pairs_taps(FORM) ? 2 * (uo % hs) + row / (SR / 2) : uo % hs;
+    const int rr = uo / hs;
     int r = rr, s = ss;
     if (p.up > 1) {
       const int rho = it.ph / p.up;
@@ -940,7 +962,8 @@ namespace {
 
 // The plan of one form, or false where the form or the kernel does not take the
 // shape.  *cost: modelled MMA cycles of the longest-running CTA.
-bool plan_form(const ConvGeom &g, int terms, int form, int sms, BankParams *out, double *cost_out) {
+// split: one input phase per halo block.
+bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, BankParams *out, double *cost_out) {
   if (g.mode != CCT_PROJECT_FRAME_BLOCK_REDUCE_SUM && g.mode != CCT_BACK_PROJECT_FRAME_BLOCK_REDUCE_SUM)
     return false;
   if (terms != 2 && terms != 3) return false;
@@ -1027,6 +1050,9 @@ bool plan_form(const ConvGeom &g, int terms, int form, int sms, BankParams *out,
         }
       }
   }
+  if (split && p.nphase == 1) return false;
+  p.hblocks = split ? p.nphase : 1;
+  const int NUP = (NU + p.hblocks - 1) / p.hblocks;  // units of a halo block, about
   // Band width BW, tile size N (positions) and plane block CB, by a cost
   // model: an M=128, 16-deep MMA over N positions takes N/2 tensor cycles and
   // reads 4 KB of filter plus 32*N bytes of halo from shared memory at about
@@ -1057,7 +1083,7 @@ bool plan_form(const ConvGeom &g, int terms, int form, int sms, BankParams *out,
       for (int CB : {64, 32, 16}) {
         if (CB > cmax && CB != 16) continue;
         const size_t part = (size_t)L * CB * 2;
-        const size_t halo = (((size_t)p.nphase * terms * part) + 127) & ~(size_t)127;
+        const size_t halo = (((size_t)(split ? 1 : p.nphase) * terms * part) + 127) & ~(size_t)127;
         const size_t chunk = (size_t)p.arows * CB * 2;
         // Units per stage: each stage hand-off (the MMA thread's wait and
         // commit, the loader's refill) costs ~400 cycles of the issuing
@@ -1069,15 +1095,19 @@ bool plan_form(const ConvGeom &g, int terms, int form, int sms, BankParams *out,
         const double tap_cycles = (CB / 16) * p.nmma * std::max(0.5 * N, 32.0 + 0.25 * N);
         auto fits = [&](int t, int st) { return 2 * halo + (size_t)st * t * chunk + xch_bytes <= budget; };
         auto ok_stages = [&](int t) { return fits(t, 3) || (fits(t, 2) && t * tap_cycles >= 1500.0); };
-        int T = std::min(NU, std::max(1, (int)(2000.0 / tap_cycles)));
+        int T = std::min(NUP, std::max(1, (int)(2000.0 / tap_cycles)));
         while (T > 1 && !ok_stages(T)) --T;
         if (!ok_stages(T) || L * 16 >= (1 << 18)) continue;
-        if (T * tap_cycles < 500.0 && T < NU && CB > 16) continue;  // a smaller plane block keeps stages long
+        if (T * tap_cycles < 500.0 && T < NUP && CB > 16) continue;  // a smaller plane block keeps stages long
         // work items run in waves over the SMs: a small problem takes smaller
         // tiles to occupy more of them
         const long long items = (long long)g.batch * p.nph_out * nbands * tiles * p.nblocks;
         const double waves = (double)((items + sms - 1) / sms);
-        const double cost = waves * (std::max(0.5 * N, 32.0 + 0.25 * N) + 8.0);
+        // a stage of less than ~500 cycles of MMAs takes that long all the same (two
+        // terms, 3x3 64 -> 64 on 8x 224x224 down 2: 80 us with 256-cycle stages of N =
+        // 256, 69 with longer ones of a smaller N)
+        const double cost =
+            waves * (std::max(0.5 * N, 32.0 + 0.25 * N) + 8.0) * std::max(1.0, 500.0 / (T * tap_cycles));
         if (!found || cost < best_cost * 0.999 || (cost <= best_cost * 1.001 && CB > best_cb)) {
           p.nbands = nbands;
           p.BW = BW;
@@ -1113,13 +1143,24 @@ bool plan_form(const ConvGeom &g, int terms, int form, int sms, BankParams *out,
     for (int tap = 0; tap < RS; ++tap) {
       const int r = tap / g.S, s = tap % g.S;
       const int ar = r - g.low_r, ac = s - g.low_c;
-      p.tap_phase[tap] = phase_of[pos_mod(ar, d)][pos_mod(ac, d)];
+      p.tap_phase[tap] = split ? 0 : phase_of[pos_mod(ar, d)][pos_mod(ac, d)];
       p.tap_off[tap] = (floor_div(ar, d) - p.sr_min) * p.P + (floor_div(ac, d) - p.sc_min);
     }
   }
   p.NCB = (g.n + p.CB - 1) / p.CB;
+  if (split) {  // units ordered by the phase they read
+    int k = 0;
+    p.nst = 0;
+    for (int ph = 0; ph < p.nphase; ++ph) {
+      p.ph_u0[ph] = k;
+      for (int tap = 0; tap < RS; ++tap)
+        if (phase_of[pos_mod(tap / g.S - g.low_r, d)][pos_mod(tap % g.S - g.low_c, d)] == ph) p.unit_tap[k++] = tap;
+      p.nst += (k - p.ph_u0[ph] + p.T - 1) / p.T;
+    }
+    p.ph_u0[p.nphase] = k;
+  }
   p.KS = p.CB / 16;
-  p.nst = (NU + p.T - 1) / p.T;
+  if (!split) p.nst = (NU + p.T - 1) / p.T;
   const int tstages = p.NCB * p.nst;
   // Promotion: the hi*hi accumulator takes at most 64 k-steps (1024 terms of
   // the reduction) before it is added into the FP32 running sum.
@@ -1157,8 +1198,8 @@ bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
   // taps of a filter row share it instead where they can.
   BankParams p{}, w{};
   double cost = 0.0, wcost = 0.0;
-  const bool paired = terms == 2 && plan_form(g, terms, kPair, sms, &p, &cost);
-  const bool ok = paired || plan_form(g, terms, kPlain, sms, &p, &cost);
+  const bool paired = terms == 2 && plan_form(g, terms, kPair, false, sms, &p, &cost);
+  const bool ok = paired || plan_form(g, terms, kPlain, false, sms, &p, &cost);
   if (!ok) return false;
   p.pack_limit = p.pack_bytes;
   // The wide forms where the model says they take fewer MMA cycles: 128 filters
@@ -1168,9 +1209,20 @@ bool bank_tc_plan(const ConvGeom &g, int terms, int sms, BankParams *out) {
   // 96 -> 85 us; 3x3 64 -> 64 on 8x 112x112, 0.83, 60 / 69 us).  Never a larger
   // packed operand: whoever holds a fixed scratch for it keeps what it takes.
   const int form = paired ? -1 : g.groups > 64 ? kWide : kWidePair;
-  if (form >= 0 && plan_form(g, terms, form, sms, &w, &wcost) && wcost < (form == kWide ? 0.95 : 0.78) * cost &&
+  if (form >= 0 && plan_form(g, terms, form, false, sms, &w, &wcost) && wcost < (form == kWide ? 0.95 : 0.78) * cost &&
       w.pack_bytes <= p.pack_bytes) {
     w.pack_limit = p.pack_bytes;
+    p = w;
+    cost = wcost;
+  }
+  // One input phase per halo block, where that lets a three-term DownsampleOutput(2)
+  // layer have longer stages: all four phases often leave room for one tap of 16
+  // planes (3x3 64 -> 64 on 8x 224x224: 129 us, 92 split; 7x7 32 -> 32 on 4x 64x64: 47 /
+  // 33).  At equal stages it loses (256 -> 256 on 56x56: 59 / 62), and in two terms,
+  // whose phases of one tap convert for longer than they multiply (80 / 96, 41 / 46).
+  if (terms == 3 && plan_form(g, terms, p.form, true, sms, &w, &wcost) && wcost < 0.97 * cost &&
+      w.pack_bytes <= p.pack_limit) {
+    w.pack_limit = p.pack_limit;
     p = w;
   }
   *out = p;

@@ -36,7 +36,11 @@ struct BankParams {
   int nphase;       // input phases held in the halo
   int phase_r[kBankMaxPhases], phase_c[kBankMaxPhases];  // row / column phase of each
   int sr_min, sc_min;  // smallest row / column shift (in strided units)
-  int tap_phase[kBankMaxTaps];  // halo phase a tap reads
+  int tap_phase[kBankMaxTaps];  // phase of its halo block that a tap reads
+  int hblocks;                  // halo blocks per plane block: 1 (all phases), or one per phase
+  // one per phase: the units (taps) ordered by the phase they read, phase ph's
+  // being [ph_u0[ph], ph_u0[ph + 1])
+  int unit_tap[kBankMaxTaps], ph_u0[kBankMaxPhases + 1];
   int tap_off[kBankMaxTaps];    // position offset of a tap inside its phase
   int tstride;                  // tap index of filter row r, column s: r * tstride + s
   // UpsampleInput(up): each output phase (rho, kappa) = (i mod up, j mod up)
@@ -50,10 +54,11 @@ struct BankParams {
   int up_sr[kBankMaxUp], up_sc[kBankMaxUp];  // input row / column of sub-tap 0 at grid position 0
   int up_choff[kBankMaxUp * kBankMaxUp];     // first packed chunk of each output phase
   uint32_t part_bytes;   // one split term of one phase: L * CB * 2
-  uint32_t halo_bytes;   // one halo buffer: nphase * terms * part_bytes
+  uint32_t halo_bytes;   // one halo buffer: terms * part_bytes of each of its phases
   uint32_t chunk_bytes;  // one packed filter chunk (one unit, one plane block): arows * CB * 2
   int T;                 // units per stage (one bulk copy of T consecutive chunks)
-  int nst;               // stages per (tile, plane block): ceil(nunits / T), the most of any phase
+  int nst;               // stages per (tile, plane block): ceil(nunits / T), the most of any
+                         // output phase; the sum over the halo blocks
   uint32_t stage_bytes;  // T * chunk_bytes
   int stages;            // stage pipeline depth
   int seg_stages;        // stages per accumulation segment

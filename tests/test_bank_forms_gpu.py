@@ -50,3 +50,14 @@ def test_forms(batch, C, K, rows, cols, R, border, sampling, step, mode, prec):
     assert np.array_equal(runs[0], runs[1]) and np.array_equal(runs[0], runs[2])
     scale = np.abs(ref).max()
     assert np.abs(runs[0] - np.maximum(ref, 0)).max() <= BOUND[prec] * scale
+
+
+# DownsampleOutput(2) in three terms with one input phase per halo block, and
+# two-term layers whose stages the plan lengthens
+@pytest.mark.parametrize("prec", [_lib.PREC_BF16X3, _lib.PREC_BF16X6])
+@pytest.mark.parametrize("batch,C,K,rows,cols,R,border", [
+    (1, 64, 64, 64, 224, 3, O.ZERO), (2, 32, 32, 40, 44, 7, O.CYCLIC), (1, 40, 50, 32, 120, 5, O.CLAMP),
+    (3, 17, 64, 18, 226, 3, O.CLAMP), (1, 128, 60, 20, 160, 5, O.ZERO), (1, 20, 20, 16, 16, 9, O.ZERO)])
+def test_down2(batch, C, K, rows, cols, R, border, prec):
+    test_forms(batch, C, K, rows, cols, R, border, O.DOWN, 2, O.PROJECT_REDUCE, prec)
+    test_forms(batch, C, K, rows, cols, R, border, O.DOWN, 2, O.BACKPROJECT_REDUCE, prec)
