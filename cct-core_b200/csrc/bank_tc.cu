@@ -79,9 +79,11 @@ constexpr int kThreads = 32 * (kEpiWarp0 + kEpiWarps);
 constexpr int kMaxStages = 8;
 constexpr int kPackThreads = 128;
 constexpr uint32_t kAccCols = 256;  // one accumulator (N <= 256 fp32 columns)
-// Epilogue exchange: eight part tiles of 32 filters x 16 positions (row
-// pitch 17 floats: conflict-free by filter and by position).
-constexpr int kXchPitch = 17;
+// Epilogue exchange: eight part tiles of 32 filters x 16 positions, a filter's
+// four float4s permuted by its number (xch_quad) so that eight filters' float4s
+// of one position, and two filters' rows, cover all banks.
+constexpr int kXchPitch = 16;
+__device__ __forceinline__ int xch_quad(int filter, int quad) { return quad ^ ((filter >> 1) & 3); }
 constexpr int kXchFloats = 32 * kXchPitch;
 constexpr size_t kXchBytes = 8 * kXchFloats * sizeof(float);
 
@@ -360,9 +362,11 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
       if (lane == 0) mbar_arrive(release);
     }
     {
-      float *mine = tiles + part * kXchFloats + lane * kXchPitch;
+      float4 *mine = reinterpret_cast<float4 *>(tiles + part * kXchFloats + lane * kXchPitch);
 #pragma unroll
-      for (int t = 0; t < 16; ++t) mine[t] = shifted ? v[t + 1] : v[t];
+      for (int k = 0; k < 4; ++k)
+        mine[xch_quad(lane, k)] = shifted ? make_float4(v[4 * k + 1], v[4 * k + 2], v[4 * k + 3], v[4 * k + 4])
+                                          : make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     }
     if (kAhead && c + 16 < cbeg + ncol) issue(c + 16);
     group_sync<G>(bar_id);  // every part of the chunk is in place
@@ -377,10 +381,14 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
 #pragma unroll
       for (int k = 0; k < 4 / G; ++k)
 #pragma unroll
-        for (int q = 0; q < G; ++q)
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            w[(k * G + q) * 4 + e] = tiles[q * kXchFloats + (8 * (part * (4 / G) + k) + fl) * kXchPitch + t0 + e];
+        for (int q = 0; q < G; ++q) {
+          const int f = 8 * (part * (4 / G) + k) + fl;
+          const float4 r = reinterpret_cast<const float4 *>(tiles + q * kXchFloats + f * kXchPitch)[xch_quad(f, lane & 3)];
+          w[(k * G + q) * 4 + 0] = r.x;
+          w[(k * G + q) * 4 + 1] = r.y;
+          w[(k * G + q) * 4 + 2] = r.z;
+          w[(k * G + q) * 4 + 3] = r.w;
+        }
     } else {
       // lane -> (filter 2*i + lane/16, position lane%16), i in the share
       t0 = lane & 15;
@@ -388,8 +396,10 @@ __device__ __forceinline__ void store_tile_columns(const BankParams &p, const It
 #pragma unroll
       for (int k = 0; k < 16 / G; ++k)
 #pragma unroll
-        for (int q = 0; q < G; ++q)
-          w[k * G + q] = tiles[q * kXchFloats + (2 * (part * (16 / G) + k) + fl) * kXchPitch + t0];
+        for (int q = 0; q < G; ++q) {
+          const int f = 2 * (part * (16 / G) + k) + fl;
+          w[k * G + q] = tiles[q * kXchFloats + f * kXchPitch + 4 * xch_quad(f, t0 >> 2) + (t0 & 3)];
+        }
     }
     group_sync<G>(bar_id);  // the tiles may be rewritten
     const int Gp = p0 + c + t0;
@@ -440,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ Bars bars;
   // epilogue exchange: 4 groups of 2 part tiles, or (paired taps) 2 groups of 4
-  __shared__ float xch[8 * kXchFloats];
+  __shared__ __align__(16) float xch[8 * kXchFloats];
   __shared__ uint32_t unit_boff[kBankMaxTaps];  // MMA warp: B operand offset of each unit
   const ConvGeom &g = p.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -761,7 +771,7 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
     group_of<FORM>(quarter, half, grp, part);
     const int bar_id = 2 + grp;
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    float *tiles = xch + grp * G * kXchFloats;  // the group's part tiles, [part][filter][pitch 17]
+    float *tiles = xch + grp * G * kXchFloats;  // the group's part tiles, [part][filter][16]
     const bool helped = helpers_store_last(p);
     uint32_t u = 0;
     bool failed = false;
