@@ -47,6 +47,11 @@ namespace {
 // columns, or more while that leaves fewer than 64 threads.
 __host__ __device__ constexpr int row_threads(int N) { return N / 16 > 64 ? N / 16 : 64; }
 __host__ __device__ constexpr int col_width(int Fr) { return Fr / 16 * 4 >= 64 ? 4 : 64 / (Fr / 16); }
+// Column threads to keep resident per SM: 1024 (64 registers a thread, a few
+// spilled) for the long columns that fill the SMs; up to 1024 rows a plane has at
+// most 129 CTAs, so 512 and no spills (512x512: 20.8 us a convolution, 18.7 so;
+// 2048x2048: 56.7, 62.0 so).
+__host__ __device__ constexpr int col_residency(int Fr) { return Fr <= 1024 ? 512 : 1024; }
 // Shared-memory stride of a column in complex values: a warp holds 32/CW
 // consecutive elements of each of CW columns, so a stride of 32/CW (mod 16)
 // spreads its 32 values evenly over the banks.
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(row_threads(1 << LOGN), 1024 / row_threads(1 <
 // MODE 1: forward FFT and scaling by p.scale of the filters' rows, into spec.
 template <int MODE, int LOGR>
 __global__ void __launch_bounds__(col_width(1 << LOGR) * (1 << LOGR) / 16,
-                                  1024 / (col_width(1 << LOGR) * (1 << LOGR) / 16))
+                                  col_residency(1 << LOGR) / (col_width(1 << LOGR) * (1 << LOGR) / 16))
     fft_cols(FftParams p, float2 *__restrict__ spec, const float2 *__restrict__ G) {
   extern __shared__ __align__(16) float2 fsm[];
   grid_dependency_wait();  // launched with programmatic serialisation
