@@ -44,9 +44,12 @@ namespace cct {
 namespace {
 
 // Threads of a row CTA (as many rows as they hold) and of a column CTA: four
-// columns, or more while that leaves fewer than 64 threads.
+// columns, or more while that leaves fewer than 64 threads; two of 4096 rows, so
+// that two CTAs share an SM (2048x2048 clamp: 171 us with one of 1024 threads, 160).
 __host__ __device__ constexpr int row_threads(int N) { return N / 16 > 64 ? N / 16 : 64; }
-__host__ __device__ constexpr int col_width(int Fr) { return Fr / 16 * 4 >= 64 ? 4 : 64 / (Fr / 16); }
+__host__ __device__ constexpr int col_width(int Fr) {
+  return Fr == 4096 ? 2 : Fr / 16 * 4 >= 64 ? 4 : 64 / (Fr / 16);
+}
 // Column threads to keep resident per SM: 1024 (64 registers a thread, a few
 // spilled) for the long columns that fill the SMs; up to 1024 rows a plane has at
 // most 129 CTAs, so 512 and no spills (512x512: 20.8 us a convolution, 18.7 so;
@@ -158,6 +161,20 @@ __device__ __forceinline__ void dft(float2 *v) {
   if (R == 16) dft16<INV>(v);
 }
 
+// Forward 16-point DFT of (a, 0, .., 0, b): a + b exp(2 pi i k / 16).
+__device__ __forceinline__ void dft16_ends(float2 a, float2 b, float2 (&v)[16]) {
+  constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508978f, h = 0.70710678118654752f;
+  constexpr float c[5] = {1.0f, c1, h, s1, 0.0f};  // cos(pi k / 8); sin(pi k / 8) = c[4 - k]
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 t = cmul(b, make_float2(c[k], c[4 - k]));
+    v[k] = cadd(a, t);
+    v[k + 8] = csub(a, t);
+    v[k + 4] = cadd(a, rot<true>(t));
+    v[k + 12] = csub(a, rot<true>(t));
+  }
+}
+
 // One Stockham pass of radix R over an N-point sequence (T = N/16 threads,
 // thread tt owns butterflies j = tt + q*T, q < 16/R): twiddles
 // w_(Ns R)^(m k) on input m (k = j mod Ns), then the R-point DFT.
@@ -219,11 +236,11 @@ __device__ __forceinline__ void pass_store(float2 *s, const float2 (&v)[16], int
 // The passes (radix 16, the last 2..16) are fixed at compile time.  Every
 // thread of the CTA takes part (the passes synchronise the CTA); SYNC: others
 // may still read s when this starts.
-template <int LOGN, bool INV, bool SYNC, int NS_LOG = 0>
+template <int LOGN, bool INV, bool SYNC, int NS_LOG = 0, bool PRE = false>
 __device__ __forceinline__ void fft_regs(float2 *s, float2 (&v)[16], int tt, const float2 *__restrict__ tw) {
   constexpr int B = (LOGN - NS_LOG) >= 4 ? 4 : (LOGN - NS_LOG);
   constexpr int R = 1 << B, N = 1 << LOGN, T = N / 16;
-  pass_compute<R, INV>(v, N, 1 << NS_LOG, T, tt, tw);
+  if (!PRE) pass_compute<R, INV>(v, N, 1 << NS_LOG, T, tt, tw);  // PRE: the caller did the first pass
   if constexpr (NS_LOG + B < LOGN) {
     constexpr int R2 = 1 << ((LOGN - NS_LOG - B) >= 4 ? 4 : (LOGN - NS_LOG - B));
     if (SYNC || NS_LOG > 0) __syncthreads();
@@ -383,16 +400,25 @@ __global__ void __launch_bounds__(col_width(1 << LOGR) * (1 << LOGR) / 16,
       const int r = tt + m * T;
       v[m] = active && (r < p.top || r >= Fr - p.bottom) ? sp[(size_t)r * 4] : make_float2(0.0f, 0.0f);
     }
+    fft_regs<LOGR, false, false>(s, v, tt, p.tw_r);
   } else {
     const ConvGeom &g = p.g;
     const float2 *rp = G + (size_t)pl * g.R * p.ld + spec_index(0, col, g.R);
+    auto row = [&](int r) {
+      const int i = filter_index(r, (g.R - 1) / 2, g.R, Fr, g.orient == CCT_CONVOLUTION);
+      return active && i >= 0 ? __ldg(rp + (size_t)i * 4) : make_float2(0.0f, 0.0f);
+    };
+    if ((g.R - 1) / 2 < T) {
+      // the filter's rows lie in the first and the last sixteenth of the grid:
+      // a thread's first DFT has two inputs that are not zero
+      dft16_ends(row(tt), row(tt + 15 * T), v);
+      fft_regs<LOGR, false, false, 0, true>(s, v, tt, p.tw_r);
+    } else {
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int i = filter_index(tt + m * T, (g.R - 1) / 2, g.R, Fr, g.orient == CCT_CONVOLUTION);
-      v[m] = active && i >= 0 ? __ldg(rp + (size_t)i * 4) : make_float2(0.0f, 0.0f);
+      for (int m = 0; m < 16; ++m) v[m] = row(tt + m * T);
+      fft_regs<LOGR, false, false>(s, v, tt, p.tw_r);
     }
   }
-  fft_regs<LOGR, false, false>(s, v, tt, p.tw_r);
   if (MODE == 0) {
     int ip, fp;
     plane_pair(p.g, pl, 0, &ip, &fp);
