@@ -1077,7 +1077,7 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
   const size_t budget = 225 * 1024;
   const int cmax = ((g.n + 15) / 16) * 16;
   bool found = false;
-  double best_cost = 0.0;
+  double best_cost = 0.0, best_waves = 0.0;
   int best_cb = 0;
   for (int bw : {p.OWq, 512, 256, 192, 128, 96, 64, 48, 32}) {
     if (bw > p.OWq || (bw == p.OWq && bw > 1024)) continue;
@@ -1140,6 +1140,7 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
           p.tile_adv = adv;
           p.tiles_band = (int)tiles;
           best_cost = cost;
+          best_waves = waves;
           best_cb = CB;
           found = true;
         }
@@ -1203,7 +1204,13 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
   }
   p.pack_bytes = chunks * p.chunk_bytes;
   *out = p;
-  *cost_out = best_cost * p.NCB * p.KS * NU * p.nmma;
+  // A tile takes its MMAs or its epilogue, whichever is longer: the epilogue about
+  // 50 cycles a position (3 -> 64 planes on 8x 224x224), 80 where it adds shifted taps.
+  double units = 0.0;
+  for (int ph = 0; ph < p.nph_out; ++ph)
+    units += u > 1 ? units_of(p.up_rq[ph / u], p.up_sq[ph % u]) : NU;
+  const double mmas = best_cost / best_waves * p.NCB * p.KS * p.nmma * units / p.nph_out;
+  *cost_out = best_waves * std::max(mmas, (p.pair ? 80.0 : 50.0) * p.N);
   return true;
 }
 

@@ -174,7 +174,7 @@ inline size_t wide_smem(int R, int S, int V) {
 }
 
 template <int S, int V>
-__global__ void __launch_bounds__(kWdThreads, V > 5 ? 4 : V > 3 ? 5 : V > 1 ? 6 : 8)
+__global__ void __launch_bounds__(kWdThreads, V > 1 ? 6 : 8)
     direct_wide_kernel(ConvGeom g, const float *__restrict__ x, const float *__restrict__ f,
                        float *__restrict__ y, int tiles_x, int tiles_y) {
   constexpr int U = kWdU, TW = kWdTW, TH = kWdTY * V, PITCH = wide_pitch(S), SP = (S + 3) & ~3;
@@ -296,7 +296,7 @@ struct UpTile {
 };
 
 template <int R, int UP, int V>
-__global__ void __launch_bounds__(kSmThreads, R == 7 || UP == 3 ? 3 : 4)
+__global__ void __launch_bounds__(kSmThreads, R == 9 ? 2 : R == 7 || UP == 3 ? 3 : 4)
     direct_up_kernel(ConvGeom g, const float *__restrict__ x, const float *__restrict__ f, float *__restrict__ y,
                      int tiles_x, int tiles_y) {
   using T = UpTile<R, UP, V>;
@@ -594,7 +594,7 @@ int launch_up_v(const ConvGeom &g, const float *x, const float *f, float *y, cud
 
 template <int R, int UP>
 int launch_up(const ConvGeom &g, const float *x, const float *f, float *y, cudaStream_t st) {
-  if constexpr (UP == 2) {
+  if constexpr (UP == 2 && R < 9) {
     const int rc = launch_up_v<R, UP, 2>(g, x, f, y, st, kTallTiles);
     if (rc != 1) return rc;
   }
@@ -668,6 +668,9 @@ int launch_direct(const ConvGeom &g, const float *x, const float *f, float *y,
   case RR: return g.up == 2 ? launch_up<RR, 2>(g, x, f, y, st) : launch_up<RR, 3>(g, x, f, y, st);
     switch (g.R) {
       CCT_UP_CASE(3) CCT_UP_CASE(5) CCT_UP_CASE(7)
+      case 9:
+        if (g.up == 2) return launch_up<9, 2>(g, x, f, y, st);
+        break;
       default: break;
     }
 #undef CCT_UP_CASE

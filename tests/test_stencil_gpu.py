@@ -161,3 +161,9 @@ def test_separable_tiles(planes, rows, cols, rl, cl, border):
     b = {"zero": C.BorderZero, "clamp": C.BorderClamp, "cyclic": C.BorderCyclic}[border]
     y = C.convolveSeparable(torch.from_numpy(x).cuda(), torch.from_numpy(rf).cuda(), torch.from_numpy(cf).cuda(), b)
     assert bitwise_equal(y.cpu().numpy(), O.separable(x, rf, cf, _BORDERS[border], O.CONV))
+
+
+@pytest.mark.parametrize("border", ["zero", "cyclic"])
+@pytest.mark.parametrize("planes,rows,cols,shift", [(1, 17, 65, 0), (3, 33, 64, 0), (2, 9, 6, 1), (1, 3, 1, 0)])
+def test_up2_9x9(planes, rows, cols, shift, border):
+    _check(rows, cols, 9, 9, border, O.CONV, planes=planes, sampling=O.UP, step=2, shift=shift)
