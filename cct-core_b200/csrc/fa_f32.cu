@@ -390,16 +390,27 @@ __global__ void __launch_bounds__(kFaThreads)
     if (s < g.OW) yp[s] = relu ? fmaxf(acc[s], 0.0f) : acc[s];
 }
 
-// out[w] = sum_b part[B*w + b], images in order (acc from 0).
-__global__ void fa_reduce_kernel(const float *__restrict__ part, float *__restrict__ y, int B, long long planes,
-                                 int plane_elems, bool relu) {
+// out[w] = sum_b part[B*w + b], images in order (acc from 0).  Bound: the latency
+// of its loads, so eight images' values are read before they are added.
+__global__ void __launch_bounds__(256) fa_reduce_kernel(const float *__restrict__ part, float *__restrict__ y, int B,
+                                                        long long planes, int plane_elems, bool relu) {
+  grid_dependency_wait();  // launched with programmatic serialisation: nothing global before this
+  allow_dependent_launch();
   const long long n = planes * plane_elems;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (long long)gridDim.x * blockDim.x) {
     const long long w = e / plane_elems, q = e - w * plane_elems;
     const float *pp = part + (size_t)w * B * plane_elems + q;
     float acc = 0.0f;
-    for (int b = 0; b < B; ++b) acc = __fadd_rn(acc, pp[(size_t)b * plane_elems]);
+    int b = 0;
+    for (; b + 8 <= B; b += 8) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = pp[(size_t)(b + i) * plane_elems];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc = __fadd_rn(acc, v[i]);
+    }
+    for (; b < B; ++b) acc = __fadd_rn(acc, pp[(size_t)b * plane_elems]);
     y[e] = relu ? fmaxf(acc, 0.0f) : acc;
   }
 }
@@ -506,8 +517,9 @@ int launch_fa_f32(const ConvGeom &g, const float *x, const float *f, float *y, f
     const long long planes = (long long)g.n * g.groups;
     const long long n = planes * g.OH * g.OW;
     const int rblocks = (int)std::min<long long>((n + 255) / 256, 148LL * 8);
-    fa_reduce_kernel<<<rblocks, 256, 0, st>>>(work, y, g.batch, planes, g.OH * g.OW,
-                                              (g.flags & CCT_FLAG_RELU) != 0);
+    int rc = launch_pdl(fa_reduce_kernel, dim3(rblocks), dim3(256), 0, st, "fa_reduce_kernel launch", work, y, g.batch,
+                        planes, g.OH * g.OW, (g.flags & CCT_FLAG_RELU) != 0);
+    if (rc) return rc;
     count_launches(1);
   }
   return check_cuda(cudaGetLastError(), "FilterAdjoint launch");
