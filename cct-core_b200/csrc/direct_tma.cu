@@ -327,10 +327,13 @@ bool direct_tma_supported(const ConvGeom &g, const float *x) {
   // Fewer than 96 of these tiles leave most SMs idle, and a field that fills
   // less than half of its tiles wastes the rest: the direct stencils' smaller
   // tiles are faster there (us, 5x5: one plane of 256x256 4.0 / 2.4, eight 4.2 /
-  // 3.7, sixteen 4.2 / 5.3; 2048 planes of 60x64 27.3 / 25.4).
-  const long long outs = padded<true>(g.OH, g.OW) < padded<false>(g.OH, g.OW) ? padded<true>(g.OH, g.OW)
-                                                                               : padded<false>(g.OH, g.OW);
-  return outs / (64 * 128) * g.pout >= 96 && outs < 2LL * g.OH * g.OW;
+  // 3.7, sixteen 4.2 / 5.3; 1024 planes of 60x64 18.9 / 13.5), unless they
+  // waste about as much (403 planes of 1174x32: 3x3 38.1 / 44.3, 7x7 86.4 / 89.5; 400 of
+  // 32x1000: 3x3 28.1 / 34.7, but 7x7, whose direct tile is 48 rows, 66.7 / 53.6).
+  const long long wide = padded<true>(g.OH, g.OW), tall = padded<false>(g.OH, g.OW), outs = wide < tall ? wide : tall;
+  const int th = g.R == 7 ? 48 : 64;
+  const long long direct = (long long)((g.OH + th - 1) / th * th) * ((g.OW + 63) / 64 * 64);
+  return outs / (64 * 128) * g.pout >= 96 && (outs < 2LL * g.OH * g.OW || outs * 10 <= direct * 11);
 }
 
 int launch_direct_tma(const ConvGeom &g, const float *x, const float *f, float *y,

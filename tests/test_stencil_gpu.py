@@ -167,3 +167,12 @@ def test_separable_tiles(planes, rows, cols, rl, cl, border):
 @pytest.mark.parametrize("planes,rows,cols,shift", [(1, 17, 65, 0), (3, 33, 64, 0), (2, 9, 6, 1), (1, 3, 1, 0)])
 def test_up2_9x9(planes, rows, cols, shift, border):
     _check(rows, cols, 9, 9, border, O.CONV, planes=planes, sampling=O.UP, step=2, shift=shift)
+
+
+# narrow or flat fields of many planes, which fill less than half of a 64 x 128 or
+# 128 x 64 tile
+@pytest.mark.parametrize("border", ["zero", "valid", "full"])
+@pytest.mark.parametrize("R", [1, 3, 5, 7])
+@pytest.mark.parametrize("planes,rows,cols", [(60, 257, 32), (100, 130, 24), (100, 32, 132), (100, 68, 68), (100, 60, 64)])
+def test_narrow(planes, rows, cols, R, border):
+    _check(rows, cols, R, R, border, O.CONV, planes=planes)
