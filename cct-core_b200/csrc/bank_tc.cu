@@ -1256,10 +1256,12 @@ int launch_bank_pack(const BankParams &p, const float *f, uint8_t *packed, cudaS
   const long long total = (long long)p.nph_out * p.nblocks * p.NCB * p.nunits * (wide_form(p.form) ? 128 : 64) * (p.CB / 8);
   if (total > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "packed filter operand too large");
   // One CTA per SM (more would wait for the filter-bank CTAs to leave) while a
-  // thread then packs one row; a larger bank takes up to 16 (3x3 256 -> 256 planes on
-  // 8x 28x28, dynamic filter: 75 us with one, 66 with more).
+  // thread then packs one or two rows; a larger bank takes up to 16 (dynamic filter,
+  // one / more, us by rows per thread: 1.1, 7x7 96 -> 32 planes on 2x 45x85 31.9 / 41.8;
+  // 1.4, 5x5 64 -> 128 on 8x 40x40 28.4 / 27.6; 1.5, 7x7 128 -> 32 39.3 / 50.9; 2.9, 3x3 192 ->
+  // 192 on 8x 28x28 47.1 / 43.4; 3.9, 256 -> 256 65.2 / 51.1).
   const long long ctas = (total + kPackThreads - 1) / kPackThreads;
-  const int blocks = (int)std::min<long long>(ctas, ctas > 1LL * p.sms ? 16LL * p.sms : p.sms);
+  const int blocks = (int)std::min<long long>(ctas, ctas > 2LL * p.sms ? 16LL * p.sms : p.sms);
   const auto kern = p.form == kPair       ? bank_pack_kernel<kPair>
                     : p.form == kWide     ? bank_pack_kernel<kWide>
                     : p.form == kWidePair ? bank_pack_kernel<kWidePair>

@@ -61,3 +61,10 @@ def test_forms(batch, C, K, rows, cols, R, border, sampling, step, mode, prec):
 def test_down2(batch, C, K, rows, cols, R, border, prec):
     test_forms(batch, C, K, rows, cols, R, border, O.DOWN, 2, O.PROJECT_REDUCE, prec)
     test_forms(batch, C, K, rows, cols, R, border, O.DOWN, 2, O.BACKPROJECT_REDUCE, prec)
+
+
+# filter operands of one to three rows per packing thread of a CTA on each SM
+@pytest.mark.parametrize("prec", [_lib.PREC_BF16X3, _lib.PREC_BF16X6])
+@pytest.mark.parametrize("C,K,R", [(84, 32, 7), (96, 32, 7), (160, 32, 7), (176, 32, 7), (96, 64, 5), (200, 64, 5)])
+def test_pack_rows(C, K, R, prec):
+    test_forms(1, C, K, 12, 19, R, O.FULL, O.NOSAMPLE, 1, O.PROJECT_REDUCE, prec)
