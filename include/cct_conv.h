@@ -197,8 +197,9 @@ int cct_conv_scalar_matrix(int32_t rows, int32_t cols, const float *image,
  * (cct_conv_output_shape of desc) with each channel saturate(v * 255)
  * rounded half to even and alpha 255, as CreateColorFieldHyperKernel writes
  * (hyperkernels/CreateColorFieldHyperKernel.scala:35-40).  Image and output
- * must be 4-byte aligned device pointers; the plan owns six planes of
- * workspace. */
+ * must be 4-byte aligned device pointers.  Square filters of 1, 3, 5 or 7
+ * without sampling on the direct path run in one kernel; for any other the
+ * plan owns six planes of workspace. */
 typedef struct cct_color_plan cct_color_plan;
 int cct_color_plan_create(const cct_conv_desc *desc, cct_color_plan **plan);
 int cct_color_plan_set_static_filter(cct_color_plan *plan, const float *host_filter);
@@ -215,8 +216,8 @@ int cct_color_plan_destroy(cct_color_plan *plan);
  * nothing: image, filter and out are the caller's device pointers; the
  * kernel's only scratch, the packed bf16 hi/lo filter operand, lives in a
  * fixed device array of 4 MiB (held by every GPU that loads the library
- * until exit).  Descriptors whose packed operand exceeds 4 MiB are rejected
- * with CCT_EINVAL; shapes the tensor-core kernel does not take return
+ * until exit).  Descriptors whose operand, packed as blocks of 64 filters
+ * (32 for paired taps), exceeds 4 MiB are rejected with CCT_EINVAL; shapes the tensor-core kernel does not take return
  * CCT_ENOTSUP.  The first call on a device looks up the array's device
  * address (cudaGetSymbolAddress) and caches it for the life of the CUDA
  * context; make that first call before any stream capture.  All calls on a
