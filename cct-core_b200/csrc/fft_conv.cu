@@ -161,20 +161,6 @@ __device__ __forceinline__ void dft(float2 *v) {
   if (R == 16) dft16<INV>(v);
 }
 
-// Forward 16-point DFT of (a, 0, .., 0, b): a + b exp(2 pi i k / 16).
-__device__ __forceinline__ void dft16_ends(float2 a, float2 b, float2 (&v)[16]) {
-  constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508978f, h = 0.70710678118654752f;
-  constexpr float c[5] = {1.0f, c1, h, s1, 0.0f};  // cos(pi k / 8); sin(pi k / 8) = c[4 - k]
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 t = cmul(b, make_float2(c[k], c[4 - k]));
-    v[k] = cadd(a, t);
-    v[k + 8] = csub(a, t);
-    v[k + 4] = cadd(a, rot<true>(t));
-    v[k + 12] = csub(a, rot<true>(t));
-  }
-}
-
 // One Stockham pass of radix R over an N-point sequence (T = N/16 threads,
 // thread tt owns butterflies j = tt + q*T, q < 16/R): twiddles
 // w_(Ns R)^(m k) on input m (k = j mod Ns), then the R-point DFT.
@@ -236,11 +222,11 @@ __device__ __forceinline__ void pass_store(float2 *s, const float2 (&v)[16], int
 // The passes (radix 16, the last 2..16) are fixed at compile time.  Every
 // thread of the CTA takes part (the passes synchronise the CTA); SYNC: others
 // may still read s when this starts.
-template <int LOGN, bool INV, bool SYNC, int NS_LOG = 0, bool PRE = false>
+template <int LOGN, bool INV, bool SYNC, int NS_LOG = 0>
 __device__ __forceinline__ void fft_regs(float2 *s, float2 (&v)[16], int tt, const float2 *__restrict__ tw) {
   constexpr int B = (LOGN - NS_LOG) >= 4 ? 4 : (LOGN - NS_LOG);
   constexpr int R = 1 << B, N = 1 << LOGN, T = N / 16;
-  if (!PRE) pass_compute<R, INV>(v, N, 1 << NS_LOG, T, tt, tw);  // PRE: the caller did the first pass
+  pass_compute<R, INV>(v, N, 1 << NS_LOG, T, tt, tw);
   if constexpr (NS_LOG + B < LOGN) {
     constexpr int R2 = 1 << ((LOGN - NS_LOG - B) >= 4 ? 4 : (LOGN - NS_LOG - B));
     if (SYNC || NS_LOG > 0) __syncthreads();
@@ -409,10 +395,16 @@ __global__ void __launch_bounds__(col_width(1 << LOGR) * (1 << LOGR) / 16,
       return active && i >= 0 ? __ldg(rp + (size_t)i * 4) : make_float2(0.0f, 0.0f);
     };
     if ((g.R - 1) / 2 < T) {
-      // the filter's rows lie in the first and the last sixteenth of the grid:
-      // a thread's first DFT has two inputs that are not zero
-      dft16_ends(row(tt), row(tt + 15 * T), v);
-      fft_regs<LOGR, false, false, 0, true>(s, v, tt, p.tw_r);
+      // the filter's rows lie in the first and the last sixteenth of the grid: a
+      // thread's first DFT has two inputs that are not zero, and the compiler
+      // drops the arithmetic on the others, whose values it knows.  The same
+      // operations as the general case below, so the same bits: a filter with
+      // rows of zeros around it gives the field that it gives without them.
+      v[0] = row(tt);
+#pragma unroll
+      for (int m = 1; m < 15; ++m) v[m] = make_float2(0.0f, 0.0f);
+      v[15] = row(tt + 15 * T);
+      fft_regs<LOGR, false, false>(s, v, tt, p.tw_r);
     } else {
 #pragma unroll
       for (int m = 0; m < 16; ++m) v[m] = row(tt + m * T);
