@@ -246,6 +246,12 @@ int plan_filter_elems(const cct_conv_plan *p, size_t *elems) {
   return CCT_OK;
 }
 
+void plan_fft_whole_grid(cct_conv_plan *p) {
+  if (p->g.border == CCT_BORDER_ZERO) return;  // those rows are zero
+  p->fft.top = p->fft.Fr;
+  p->fft.bottom = 0;
+}
+
 }  // namespace cct
 
 extern "C" {

@@ -152,6 +152,11 @@ int record_plan_layer(const cct_conv_plan *p, RecordLayer *out);
 int plan_record_parts(const cct_conv_plan *p, cct_conv_desc *desc, const float **dev_filter, size_t *elems,
                       int *device);
 int plan_filter_elems(const cct_conv_plan *p, size_t *elems);
+// An FFT plan transforms every row of its grid from now on, also those between
+// the border below the field and the one above it, which no output depends on but
+// by rounding.  A ColorField's bytes are rounded from the result, and stay those
+// of the whole transform.  No effect on other plans.
+void plan_fft_whole_grid(cct_conv_plan *p);
 int launch_scalar_matrix(int rows, int cols, const float *x, const float *mats, int L, int size, int border,
                          float *y, cudaStream_t stream);
 int launch_separable(int rows, int cols, int planes, const float *x,

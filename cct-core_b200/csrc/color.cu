@@ -248,6 +248,7 @@ int cct_color_plan_create(const cct_conv_desc *desc, cct_color_plan **out) {
   if (!rc) rc = resolve_geom(&d, &p->g);
   int32_t algo = -1;
   if (!rc) rc = cct_conv_plan_algo(p->planes, &algo);
+  if (!rc) plan_fft_whole_grid(p->planes);
   p->fused = !rc && algo == 0 && color_fused(p->g);
   if (!rc && p->fused) {
     *out = p;
