@@ -215,6 +215,7 @@ struct cct_color_plan {
   cct_conv_plan *planes;  // the plane plan over red, green, blue
   bool fused;             // one kernel from bytes to bytes
   ConvGeom g;
+  uchar4 *copy;           // fused: a copy of the image, read where the output overlaps it
   float *in, *out;        // 3 planes each (not fused)
   long long n_in, n_out;  // pixels per plane
 };
@@ -250,7 +251,12 @@ int cct_color_plan_create(const cct_conv_desc *desc, cct_color_plan **out) {
   if (!rc) rc = cct_conv_plan_algo(p->planes, &algo);
   if (!rc) plan_fft_whole_grid(p->planes);
   p->fused = !rc && algo == 0 && color_fused(p->g);
-  if (!rc && p->fused) {
+  if (p->fused) {
+    rc = check_cuda(cudaMalloc(&p->copy, p->n_in * sizeof(uchar4)), "cudaMalloc(colour image copy)");
+    if (rc) {
+      cct_color_plan_destroy(p);
+      return rc;
+    }
     *out = p;
     return CCT_OK;
   }
@@ -267,6 +273,7 @@ int cct_color_plan_create(const cct_conv_desc *desc, cct_color_plan **out) {
 int cct_color_plan_destroy(cct_color_plan *p) {
   if (!p) return CCT_OK;
   cct_conv_plan_destroy(p->planes);
+  cudaFree(p->copy);
   cudaFree(p->in);
   cudaFree(p->out);
   delete p;
@@ -293,8 +300,16 @@ int cct_color_run(const cct_color_plan *p, const uint8_t *image, const float *fi
     if (rc) return rc;
     if (!filter) filter = dev_filter;
     if (!filter) return set_error(CCT_EINVAL, "null image, filter or output pointer");
-    return launch_color_fused(p->g, reinterpret_cast<const uchar4 *>(image), filter, reinterpret_cast<uchar4 *>(out),
-                              st);
+    const uchar4 *x = reinterpret_cast<const uchar4 *>(image);
+    // A CTA reads the halo of its tile while others store theirs: an image that
+    // the output overlaps is read from a copy.
+    if (image < out + 4 * p->n_out && out < image + 4 * p->n_in) {
+      rc = check_cuda(cudaMemcpyAsync(p->copy, x, p->n_in * sizeof(uchar4), cudaMemcpyDeviceToDevice, st),
+                      "colour image copy");
+      if (rc) return rc;
+      x = p->copy;
+    }
+    return launch_color_fused(p->g, x, filter, reinterpret_cast<uchar4 *>(out), st);
   }
   color_unpack_kernel<<<grid_for(p->n_in), 256, 0, st>>>(p->n_in, reinterpret_cast<const uchar4 *>(image), p->in);
   count_launches(1);

@@ -197,9 +197,10 @@ int cct_conv_scalar_matrix(int32_t rows, int32_t cols, const float *image,
  * (cct_conv_output_shape of desc) with each channel saturate(v * 255)
  * rounded half to even and alpha 255, as CreateColorFieldHyperKernel writes
  * (hyperkernels/CreateColorFieldHyperKernel.scala:35-40).  Image and output
- * must be 4-byte aligned device pointers.  Square filters of 1, 3, 5 or 7
- * without sampling on the direct path run in one kernel; for any other the
- * plan owns six planes of workspace. */
+ * must be 4-byte aligned device pointers and may overlap.  Square filters of
+ * 1, 3, 5 or 7 without sampling on the direct path run in one kernel, and the
+ * plan owns a copy of the image for outputs that overlap it; for any other
+ * filter the plan owns six planes of workspace. */
 typedef struct cct_color_plan cct_color_plan;
 int cct_color_plan_create(const cct_conv_desc *desc, cct_color_plan **plan);
 int cct_color_plan_set_static_filter(cct_color_plan *plan, const float *host_filter);
