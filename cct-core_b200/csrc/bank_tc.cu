@@ -60,8 +60,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
-#include <unordered_map>
 
 #include "bank_tc.h"
 #include "sm100_util.cuh"
@@ -935,29 +933,12 @@ __global__ void __launch_bounds__(kPackThreads, 16) bank_pack_kernel(const __gri
   }
 }
 
-std::mutex g_bank_mu;
-std::unordered_map<uint64_t, size_t> g_bank_attr;
-
 template <int TERMS, int FORM, bool CB16>
 int launch_terms(const BankParams &p, cudaStream_t st) {
   auto kern = bank_tc_kernel<TERMS, FORM, CB16>;
-  {
-    // Dynamic shared memory above 48 KB needs the opt-in attribute; keep the
-    // largest size set so far per (device, instance).
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t key = ((uint64_t)dev << 32) | (uint64_t)(TERMS * 8 + FORM * 2 + (CB16 ? 1 : 0));
-    std::lock_guard<std::mutex> lk(g_bank_mu);
-    size_t &have = g_bank_attr[key];
-    if (have < p.smem_bytes) {
-      const int rc = check_cuda(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)p.smem_bytes),
-                                "cudaFuncSetAttribute(bank_tc)");
-      if (rc) return rc;
-      have = p.smem_bytes;
-    }
-  }
-  const int rc = launch_pdl(kern, dim3(p.grid), dim3(kThreads), p.smem_bytes, st, "bank_tc_kernel launch", p);
+  int rc = raise_smem_limit(kern, p.smem_bytes, "cudaFuncSetAttribute(bank_tc)");
+  if (rc) return rc;
+  rc = launch_pdl(kern, dim3(p.grid), dim3(kThreads), p.smem_bytes, st, "bank_tc_kernel launch", p);
   if (rc) return rc;
   count_launches(1);
   return check_cuda(cudaGetLastError(), "bank_tc_kernel launch");

@@ -67,6 +67,21 @@ unsigned *device_error_word() {
   return g_err_word[dev];
 }
 
+int raise_smem_limit(const void *kernel, size_t bytes, const char *what) {
+  if (bytes <= 48 * 1024) return CCT_OK;
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, size_t> limits;  // by kernel and device
+  int dev = 0;
+  int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  if (rc) return rc;
+  std::lock_guard<std::mutex> lk(mu);
+  size_t &limit = limits[{kernel, dev}];
+  if (limit >= bytes) return CCT_OK;
+  rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), what);
+  if (!rc) limit = bytes;
+  return rc;
+}
+
 // Resolve and validate a descriptor.  Returns CCT_OK or CCT_EINVAL with the
 // reference's error text.
 static int resolve(const cct_conv_desc *d, ConvGeom *g) {

@@ -116,6 +116,16 @@ int launch_fa_tc(const ConvGeom &g, const float *x, const float *f, float *y, fl
 bool frame_f32_supported(const ConvGeom &g);
 int launch_frame_f32(const ConvGeom &g, const float *x, const float *f,
                      float *y, cudaStream_t stream);
+// Raises a kernel's dynamic shared-memory limit on the current device to at least
+// `bytes` (nothing to do up to 48 KB); never lowers it.  The limit belongs to the
+// kernel, not to a launch, and its sizes depend on the call: set to each call's own
+// size, a thread about to launch a large one could have it lowered by another
+// thread's small one.
+int raise_smem_limit(const void *kernel, size_t bytes, const char *what);
+template <typename... Params>
+int raise_smem_limit(void (*kernel)(Params...), size_t bytes, const char *what) {
+  return raise_smem_limit(reinterpret_cast<const void *>(kernel), bytes, what);
+}
 // Launch with programmatic stream serialisation: the kernel may be scheduled
 // while the previous kernel in the stream runs, and must call
 // grid_dependency_wait() (sm100_util.cuh) before it touches global memory

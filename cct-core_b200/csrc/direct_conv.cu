@@ -554,12 +554,8 @@ int launch_wide_v(const ConvGeom &g, const float *x, const float *f, float *y, c
   if (rc) return rc;
   if (blocks < min_blocks) return 1;  // a shorter tile is wanted
   const size_t smem = wide_smem(g.R, S, V);
-  if (smem > 48 * 1024) {
-    rc = check_cuda(cudaFuncSetAttribute(direct_wide_kernel<S, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem),
-                    "cudaFuncSetAttribute(direct_wide)");
-    if (rc) return rc;
-  }
+  rc = raise_smem_limit(direct_wide_kernel<S, V>, smem, "cudaFuncSetAttribute(direct_wide)");
+  if (rc) return rc;
   rc = launch_pdl(direct_wide_kernel<S, V>, dim3((unsigned)blocks), dim3(kWdThreads), smem, st,
                   "direct_wide_kernel launch", g, x, f, y, tx, ty);
   if (!rc) count_launches(1);
@@ -614,15 +610,11 @@ int launch_generic(const ConvGeom &g, const float *x, const float *f, float *y,
   if (smem > (size_t)max_smem)
     return set_error(CCT_ENOTSUP, "filter %dx%d with step %d needs %zu bytes of shared memory (max %d)",
                      g.R, g.S, g.down, smem, max_smem);
-  if (smem > 48 * 1024) {
-    int rc = check_cuda(cudaFuncSetAttribute(direct_generic_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                        "cudaFuncSetAttribute");
-    if (rc) return rc;
-  }
+  int rc = raise_smem_limit(direct_generic_kernel, smem, "cudaFuncSetAttribute(direct_generic)");
+  if (rc) return rc;
   const long long blocks = (long long)tiles_x * tiles_y * g.pout;
   if (blocks > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "direct convolution grid too large");
-  const int rc = launch_pdl(direct_generic_kernel, dim3((unsigned)blocks), dim3(kThreads), smem, st,
+  rc = launch_pdl(direct_generic_kernel, dim3((unsigned)blocks), dim3(kThreads), smem, st,
                             "direct_generic_kernel launch", g, x, f, y, tiles_x, tiles_y, in_rows, in_cols, pitch);
   if (!rc) count_launches(1);
   return rc;

@@ -453,12 +453,9 @@ int launch_fa_f32(const ConvGeom &g, const float *x, const float *f, float *y, f
 #define CCT_FA_QUAD_CASE(SS)                                                                                  \
   case SS: {                                                                                                  \
     const auto kern = nw == 16 ? fa_quad_kernel<SS, 16> : nw == 8 ? fa_quad_kernel<SS, 8> : fa_quad_kernel<SS, 4>; \
-    if (qsmem > 48 * 1024) {                                                                                  \
-      int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsmem), \
-                          "cudaFuncSetAttribute(fa quad)");                                                   \
-      if (rc) return rc;                                                                                      \
-    }                                                                                                         \
-    int rc = launch_pdl(kern, dim3((unsigned)qblocks), dim3(nw * 32), qsmem, st,                              \
+    int rc = raise_smem_limit(kern, qsmem, "cudaFuncSetAttribute(fa quad)");                                  \
+    if (rc) return rc;                                                                                        \
+    rc = launch_pdl(kern, dim3((unsigned)qblocks), dim3(nw * 32), qsmem, st,                              \
                         "fa_quad_kernel launch", q, x, f, dst, (int)mgroups, (int)qlgroups);                  \
     if (rc) return rc;                                                                                        \
     break;                                                                                                    \
@@ -477,12 +474,8 @@ int launch_fa_f32(const ConvGeom &g, const float *x, const float *f, float *y, f
     const int threads = kCG * kLG * g.OH;
 #define CCT_FA_ROWS_CASE(SS)                                                                            \
   case SS: {                                                                                            \
-    if (rsmem > 48 * 1024) {                                                                            \
-      int rc = check_cuda(cudaFuncSetAttribute(fa_rows_kernel<SS>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                               (int)rsmem),                                             \
-                          "cudaFuncSetAttribute(fa rows)");                                             \
-      if (rc) return rc;                                                                                \
-    }                                                                                                   \
+    int rc = raise_smem_limit(fa_rows_kernel<SS>, rsmem, "cudaFuncSetAttribute(fa rows)");              \
+    if (rc) return rc;                                                                                  \
     fa_rows_kernel<SS><<<(unsigned)rblocks, threads, rsmem, st>>>(q, x, f, dst, cgroups, lgroups);      \
     break;                                                                                              \
   }
@@ -496,12 +489,8 @@ int launch_fa_f32(const ConvGeom &g, const float *x, const float *f, float *y, f
   } else {
 #define CCT_FA_CASE(SS)                                                                               \
   case SS: {                                                                                          \
-    if (smem > 48 * 1024) {                                                                           \
-      int rc = check_cuda(cudaFuncSetAttribute(fa_f32_kernel<SS>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                               (int)smem),                                            \
-                          "cudaFuncSetAttribute(fa)");                                                \
-      if (rc) return rc;                                                                              \
-    }                                                                                                 \
+    int rc = raise_smem_limit(fa_f32_kernel<SS>, smem, "cudaFuncSetAttribute(fa)");                   \
+    if (rc) return rc;                                                                                \
     fa_f32_kernel<SS><<<(unsigned)blocks, per * g.OH, smem, st>>>(q, x, f, dst, cgroups);             \
     break;                                                                                            \
   }

@@ -840,8 +840,7 @@ int launch_fa_bank(FaBankParams p, bool conv, const float *x, const float *f, fl
   rc = encode_tensor_map_f32(&omap, p.part, 4, odims, ostr, obox);
   if (rc) return rc;
   auto kern = conv ? fa_bank_kernel<true> : fa_bank_kernel<false>;
-  rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem),
-                  "cudaFuncSetAttribute(fa_bank)");
+  rc = raise_smem_limit(kern, p.smem, "cudaFuncSetAttribute(fa_bank)");
   if (rc) return rc;
   const long long grid = (long long)p.cblocks * p.lblocks * (p.npairs * p.P + p.Q);
   rc = launch_pdl(kern, dim3((unsigned)grid), dim3(kFbThreads), p.smem, st, "fa_bank_kernel launch", p, gmap, xmap,
@@ -885,8 +884,7 @@ int launch_fa_tc(const ConvGeom &g, const float *x, const float *f, float *y, fl
   const size_t smem = 96 * 1024;
   static_assert(kStages * 2u * kNT * kKC * 2 <= 96 * 1024, "FilterAdjoint stages");
   static_assert(2 * kNT + kStages * kKC <= kTmemCols, "FilterAdjoint tensor memory");
-  int rc = check_cuda(cudaFuncSetAttribute(fa_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "cudaFuncSetAttribute(fa_tc)");
+  int rc = raise_smem_limit(fa_tc_kernel, smem, "cudaFuncSetAttribute(fa_tc)");
   if (rc) return rc;
   rc = launch_pdl(fa_tc_kernel, dim3((unsigned)grid), dim3(kFaThreads), smem, st, "fa_tc_kernel launch", p);
   if (rc) return rc;

@@ -489,14 +489,6 @@ int ilog2(int v) {
 }
 int pow2_at_least(int v) { return 1 << ilog2(v); }
 
-template <typename K>
-int set_smem(K kern, size_t bytes) {
-  if (bytes <= 48 * 1024) return CCT_OK;
-  return check_cuda(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)bytes),
-                    "cudaFuncSetAttribute(fft)");
-}
-
 // One-dimensional forward FFT of length n in FP64 (iterative radix-2, natural
 // order) of v[0], v[stride], ...; w[k] = exp(-2 pi i k / n), k < n/2.
 void fft64(std::complex<double> *v, int n, int stride, const std::vector<std::complex<double>> &w,
@@ -651,7 +643,7 @@ template <int MODE, int L>
 int launch_cols_t(const FftParams &p, float2 *spec, const float2 *G, int planes, cudaStream_t st) {
   constexpr int Fr = 1 << L, cw = col_width(Fr);
   const size_t smem = sizeof(float2) * (size_t)cw * col_stride(Fr);
-  int rc = set_smem(fft_cols<MODE, L>, smem);
+  int rc = raise_smem_limit(fft_cols<MODE, L>, smem, "cudaFuncSetAttribute(fft)");
   if (rc) return rc;
   const int cblocks = (p.Fc / 2 + 1 + cw - 1) / cw;
   rc = launch_pdl(fft_cols<MODE, L>, dim3(cblocks * planes), dim3(cw * Fr / 16), smem, st, "fft_cols launch", p, spec,
@@ -680,7 +672,7 @@ int launch_r2c_t(const FftParams &p, const float *x, const float *f, float2 *spe
   unsigned blocks;
   size_t smem;
   row_shape<L>((long long)planes * (p.top + p.bottom) + (long long)fplanes * p.g.R, &blocks, &smem);
-  int rc = set_smem(fft_rows_r2c<L>, smem);
+  int rc = raise_smem_limit(fft_rows_r2c<L>, smem, "cudaFuncSetAttribute(fft)");
   if (rc) return rc;
   rc = launch_pdl(fft_rows_r2c<L>, dim3(blocks), dim3(row_threads(1 << L)), smem, st, "fft_rows_r2c launch", p, x, f,
                   spec, rows, planes, fplanes);
@@ -694,7 +686,7 @@ int launch_c2r_t(const FftParams &p, const float2 *spec, float *y, cudaStream_t 
   unsigned blocks;
   size_t smem;
   row_shape<L>((long long)planes * p.g.OH, &blocks, &smem);
-  int rc = set_smem(fft_rows_c2r<L>, smem);
+  int rc = raise_smem_limit(fft_rows_c2r<L>, smem, "cudaFuncSetAttribute(fft)");
   if (rc) return rc;
   rc = launch_pdl(fft_rows_c2r<L>, dim3(blocks), dim3(row_threads(1 << L)), smem, st, "fft_rows_c2r launch", p, spec, y,
                   planes);

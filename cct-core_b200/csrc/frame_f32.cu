@@ -269,12 +269,9 @@ int launch_k(const ConvGeom &g, const float *x, const float *f, float *y, cudaSt
   const long long blocks = (long long)tiles_x * tiles_y * kblocks * nchunks * g.batch;
   if (blocks > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "frame grid too large");
   const auto kern = frame_f32_kernel<R, S, DOWN, REDUCE, KT, KG>;
-  if (T::SMEM > 48 * 1024) {
-    const int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM),
-                              "cudaFuncSetAttribute(frame_f32)");
-    if (rc) return rc;
-  }
-  const int rc = launch_pdl(kern, dim3((unsigned)blocks), dim3(T::THREADS), T::SMEM, st,
+  int rc = raise_smem_limit(kern, T::SMEM, "cudaFuncSetAttribute(frame_f32)");
+  if (rc) return rc;
+  rc = launch_pdl(kern, dim3((unsigned)blocks), dim3(T::THREADS), T::SMEM, st,
                             "frame_f32_kernel launch", g, x, f, y, tiles_x, tiles_y, kblocks, tchunk);
   if (!rc) count_launches(1);
   return rc;

@@ -44,8 +44,6 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <mutex>
-#include <unordered_map>
 
 #include "cct_internal.h"
 #include "frame_tc.h"
@@ -548,8 +546,6 @@ __global__ void pack_filters_kernel(ConvGeom g, const float *__restrict__ f, uin
   }
 }
 
-std::mutex g_tc_mu;
-std::unordered_map<uint64_t, size_t> g_tc_attr;
 
 template <int CB>
 int launch_cb(const TcParams &p0, const float *x, cudaStream_t st) {
@@ -559,22 +555,8 @@ int launch_cb(const TcParams &p0, const float *x, cudaStream_t st) {
   if (rc) return rc;
   const size_t smem = 2 * (size_t)p.halo_bytes + (size_t)kStages * 2u * p.NT * CB * 2;
   auto kern = frame_tc_kernel<CB>;
-  {
-    // Dynamic shared memory above 48 KB needs the opt-in attribute; keep the
-    // largest size set so far per (device, instance).
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t key = ((uint64_t)dev << 32) | (uint64_t)CB;
-    std::lock_guard<std::mutex> lk(g_tc_mu);
-    size_t &have = g_tc_attr[key];
-    if (have < smem) {
-      rc = check_cuda(cudaFuncSetAttribute((const void *)kern,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "cudaFuncSetAttribute(frame_tc)");
-      if (rc) return rc;
-      have = smem;
-    }
-  }
+  rc = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(frame_tc)");
+  if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

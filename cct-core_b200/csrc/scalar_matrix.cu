@@ -136,11 +136,8 @@ int launch_sm(int rows, int cols, const float *x, const float *mats, int L, int 
   const size_t smem = sizeof(float) * ((size_t)t.IR * t.IC + (size_t)lb * taps);
   if (smem > 200 * 1024) return set_error(CCT_ENOTSUP, "scalar-matrix convolution: matrix size %d too large", size);
   auto kern = scalar_matrix_kernel<F>;
-  if (smem > 48 * 1024) {
-    int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                        "cudaFuncSetAttribute(scalar_matrix)");
-    if (rc) return rc;
-  }
+  int rc = raise_smem_limit(kern, smem, "cudaFuncSetAttribute(scalar_matrix)");
+  if (rc) return rc;
   kern<<<dim3((unsigned)tiles, (unsigned)ly), kThreads, smem, st>>>(rows, cols, x, mats, L, size, border, y,
                                                                      tiles_x, (int)lb);
   count_launches(1);

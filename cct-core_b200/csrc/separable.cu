@@ -264,13 +264,9 @@ int launch_tile_v(int rows, int cols, int planes, const float *x, const float *r
   if (blocks < min_blocks) return 1;  // a shorter tile is wanted
   if (blocks > 0x7fffffffLL) return set_error(CCT_ENOTSUP, "separable: grid too large");
   const size_t smem = tile_smem(RL, clen, V);
-  if (smem > 48 * 1024) {
-    const int rc = check_cuda(cudaFuncSetAttribute(separable_tile<RL, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem),
-                              "cudaFuncSetAttribute(separable_tile)");
-    if (rc) return rc;
-  }
-  const int rc = launch_pdl(separable_tile<RL, V>, dim3((unsigned)blocks), dim3(kTlThreads), smem, st,
+  int rc = raise_smem_limit(separable_tile<RL, V>, smem, "cudaFuncSetAttribute(separable_tile)");
+  if (rc) return rc;
+  rc = launch_pdl(separable_tile<RL, V>, dim3((unsigned)blocks), dim3(kTlThreads), smem, st,
                             "separable launch", rows, cols, x, rf, cf, clen, border, orient, y, tx, ty);
   if (!rc) count_launches(1);
   return rc;
@@ -516,12 +512,8 @@ int launch_separable(int rows, int cols, int planes, const float *x, const float
     if (rlen <= kTlMaxR && clen <= kTlMaxC)
       return launch_tile(rows, cols, planes, x, rf, rlen, cf, clen, border, orient, y, st);
     if (blocks <= 0x7fffffffLL) {
-      if (fsmem > 48 * 1024) {
-        int rc = check_cuda(cudaFuncSetAttribute(separable_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)fsmem),
-                            "cudaFuncSetAttribute(separable)");
-        if (rc) return rc;
-      }
+      int rc = raise_smem_limit(separable_fused, fsmem, "cudaFuncSetAttribute(separable)");
+      if (rc) return rc;
       separable_fused<<<(unsigned)blocks, kThreads, fsmem, st>>>(rows, cols, planes, x, rf, rlen, cf, clen,
                                                                  border, orient, y, tiles_x, tiles_y);
       count_launches(1);
