@@ -144,7 +144,7 @@ _raw_stream = torch._C._cuda_getCurrentRawStream
 
 def _call_key(field, filt, *rest):
     return (type(field), type(filt), field.dtype, filt.dtype, field.shape, filt.shape, field.get_device(),
-            filt.get_device(), *rest)
+            filt.get_device(), rest)
 
 
 def _remember(table, key, entry):
@@ -156,8 +156,9 @@ def _remember(table, key, entry):
 def _run(field, filt, border, orientation, sampling, mode, batch, precision=_lib.PREC_FP32,
          algo=_lib.ALGO_AUTO, relu=False):
     try:
+        # the comparisons refuse a complex option, which equals an integer and hashes like it
         key = _call_key(field, filt, border.code, orientation, sampling.code, sampling.step, mode, batch, precision,
-                        algo, bool(relu))
+                        algo, bool(relu), orientation < 0, batch < 0, precision < 0)
         call = _CALLS.get(key)
     except (AttributeError, TypeError):
         key = call = None  # not tensors, or an unhashable argument: the checks below say which
