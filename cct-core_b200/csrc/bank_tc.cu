@@ -647,10 +647,10 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
         table_key = iu.ts * 1024 + iu.nu;
       }
       const int tstages = p.NCB * iu.nst;
-      int seg_left = 0, done = 0, bi = 0;
+      int seg_left = 0, done = 0, bi = 0, small_left = 0;
       // first: the next MMA starts a segment's (big) sum; first_small, wide forms:
-      // it starts the small sums, which stay in their columns for the whole item
-      // (a 2^-8 part of the result: their accumulation needs no promotion)
+      // it starts the small sums, which stay in their columns for small_segs
+      // segments (plan_form says why)
       bool first = false, first_small = true;
       for (int blk = 0; blk < p.NCB * p.hblocks && !failed; ++blk, ++hb) {
         const Block bk = block_of(p, iu, blk);
@@ -669,6 +669,11 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
             tc_fence_after();
             seg_left = min(p.seg_stages, tstages - done);
             first = true;
+            if (small_left == 0) {
+              small_left = p.small_segs;
+              first_small = true;
+            }
+            --small_left;
           }
           failed = __any_sync(0xffffffffu, !mbar_wait(&bars.full[s], sph, p.err));
           if (failed) break;
@@ -795,13 +800,21 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
         const uint32_t rc = tmem + lane_base + kAccCols;  // running sum (promotion)
         const bool first = seg == 0, last = seg == nseg - 1;
         if (!last) {
-          // promotion: R (+)= S, FP32 round to nearest, over the warp's column half
+          // promotion: R (+)= S, FP32 round to nearest, over the warp's column half;
+          // the small sums of a wide form with it where their segments end
+          const bool small = wide_form(FORM) && (seg + 1) % p.small_segs == 0;
           for (int c = half * (p.N / 2); c < (half + 1) * (p.N / 2); c += 16) {
             uint32_t s16[16], r16[16];
             tmem_ld16(sc + c, s16);
             if (!first) tmem_ld16(rc + c, r16);
             tc_wait_ld();
             if (!first) {
+#pragma unroll
+              for (int t = 0; t < 16; ++t) s16[t] = __float_as_uint(__uint_as_float(s16[t]) + __uint_as_float(r16[t]));
+            }
+            if (small) {
+              tmem_ld16(sc + kAccCols / 2 + c, r16);
+              tc_wait_ld();
 #pragma unroll
               for (int t = 0; t < 16; ++t) s16[t] = __float_as_uint(__uint_as_float(s16[t]) + __uint_as_float(r16[t]));
             }
@@ -1165,6 +1178,18 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
   const int kmax = 64;
   p.promote = p.NCB * NU * p.KS > kmax ? 1 : 0;
   p.seg_stages = p.promote ? std::max(1, kmax / (p.T * p.KS)) : tstages;
+  if (p.promote) {
+    // as many segments as that takes, of equal length: the error of a segment grows
+    // with its length (1.46e-8 of the result per k-step of three terms), so 48 + 48 + 48
+    // loses less than 64 + 64 + 16 (256 -> 192 planes, 3x3: 7.0e-7 against 9.3e-7 RMS)
+    const int nseg = (tstages + p.seg_stages - 1) / p.seg_stages;
+    p.seg_stages = (tstages + nseg - 1) / nseg;
+  }
+  // The small sums of the wide forms are a 2^-8 part of the result and could take 2^8
+  // times the MMAs of a segment for the same error; they are promoted within 2^4 times,
+  // every 1280 MMAs at most (0.3 % of the error; left in the accumulator for the
+  // whole of 6400 k-steps they raised it by a quarter).
+  p.small_segs = std::max(1, 1280 / (p.seg_stages * p.T * p.KS * (p.nmma - 1)));
   // float4 stores: groups of 4 grid positions (p0, N and tile_adv are multiples of 4)
   // never straddle a grid row or the band's last output column, and land on
   // 16-byte aligned outputs

@@ -62,6 +62,7 @@ struct BankParams {
   uint32_t stage_bytes;  // T * chunk_bytes
   int stages;            // stage pipeline depth
   int seg_stages;        // stages per accumulation segment
+  int small_segs;        // wide forms: segments per promotion of the small sums
   int promote;           // 1: segments are promoted into an FP32 running sum
   int vec4;              // 1: groups of 4 positions map to 4 aligned consecutive outputs (float4 stores)
   int grid;              // persistent CTAs
