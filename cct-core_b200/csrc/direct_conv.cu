@@ -19,7 +19,7 @@ namespace cct {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kTX = 16, kTY = 16;  // thread grid of the generic kernel
+constexpr int kTX = 16, kTY = 16;  // thread grid of the square and the generic kernel
 
 // ---------------------------------------------------------------------------
 // Small square filters (weights in registers), down-sampling 1 or 2, every
@@ -424,6 +424,111 @@ __global__ void __launch_bounds__(kSmThreads, R == 9 ? 2 : R == 7 || UP == 3 ? 3
   }
 }
 
+// ---------------------------------------------------------------------------
+// Squares over a zero-inserted grid that direct_up_kernel does not take
+// (UpsampleInput by 4 and more, BorderFull and BorderValid, 1x1): weights in
+// registers, 64 x 64 outputs a CTA, 4 x 4 a thread, the grid staged as it stands.
+// Bound: the staging, a division and a border mapping per staged value, which
+// is why 256 threads share a tile: 128 with twice the outputs took 1.2 to 2 times
+// as long, the general kernel below up to 2.7 (7x7 step 5, 569x620: 81 us here,
+// 119, 216).
+template <int R>
+__global__ void __launch_bounds__(kThreads)
+    direct_square_kernel(ConvGeom g, const float *__restrict__ x, const float *__restrict__ f,
+                         float *__restrict__ y, int tiles_x, int tiles_y) {
+  grid_dependency_wait();  // launched with programmatic serialisation: nothing global before this
+  constexpr int S = R, U = 4, V = 4, TW = kTX * U, TH = kTY * V;
+  constexpr int IN_COLS = TW - 1 + S;
+  constexpr int IN_ROWS = TH - 1 + R;
+  constexpr int PITCH = (IN_COLS + 3) & ~3;
+  constexpr int E = U - 1 + S;  // values per tile row per thread
+  constexpr int E4 = (E + 3) / 4;
+  __shared__ __align__(16) float tile[IN_ROWS * PITCH];
+
+  int bid = blockIdx.x;
+  const int tx_i = bid % tiles_x;
+  bid /= tiles_x;
+  const int ty_i = bid % tiles_y;
+  const int o = bid / tiles_y;
+  const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
+  const int out_r0 = ty_i * TH, out_c0 = tx_i * TW;
+  const int org_r = out_r0 - g.low_r;
+  const int org_c = out_c0 - g.low_c;
+
+  float acc[V][U];
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc[v][u] = 0.0f;
+
+  for (int t = 0; t < g.terms; ++t) {
+    int ip, fp;
+    plane_pair(g, o, t, &ip, &fp);
+    const float *xs = x + (size_t)ip * g.H * g.W;
+    const float *fs = f + (size_t)fp * (R * S);
+    float w[R][S];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+        w[r][s] = __ldg(fs + (g.orient == CCT_CONVOLUTION ? (R - 1 - r) * S + (S - 1 - s) : r * S + s));
+    if (t > 0) __syncthreads();
+    load_tile(tile, PITCH, IN_ROWS, IN_COLS, xs, g, org_r, org_c);
+    __syncthreads();
+
+    float rs[V][U];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int u = 0; u < U; ++u) rs[v][u] = 0.0f;
+
+    const float *base = tile + (ty * V) * PITCH + tx * U;
+#pragma unroll
+    for (int tr = 0; tr < V - 1 + R; ++tr) {
+      float vals[E4 * 4];
+#pragma unroll
+      for (int e = 0; e < E4; ++e) {
+        const float4 q = *reinterpret_cast<const float4 *>(base + tr * PITCH + 4 * e);
+        vals[4 * e + 0] = q.x;
+        vals[4 * e + 1] = q.y;
+        vals[4 * e + 2] = q.z;
+        vals[4 * e + 3] = q.w;
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int r = tr - v;
+        if (r >= 0 && r < R) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            float cs = 0.0f;
+#pragma unroll
+            for (int s = 0; s < S; ++s) cs = __fmaf_rn(vals[u + s], w[r][s], cs);
+            rs[v][u] = __fadd_rn(rs[v][u], cs);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        acc[v][u] = (t == 0) ? rs[v][u] : __fadd_rn(acc[v][u], rs[v][u]);
+  }
+
+  float *ys = y + (size_t)o * g.OH * g.OW;
+  const bool relu = (g.flags & CCT_FLAG_RELU) != 0;
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int row = out_r0 + ty * V + v;
+    if (row >= g.OH) continue;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int col = out_c0 + tx * U + u;
+      if (col < g.OW) ys[(size_t)row * g.OW + col] = relu ? fmaxf(acc[v][u], 0.0f) : acc[v][u];
+    }
+  }
+}
+
 // Any filter size and down-sampling step: filter staged in shared memory,
 // four outputs along a row per thread.
 constexpr int kGU = 4;                       // outputs per thread (columns)
@@ -597,6 +702,18 @@ int launch_up(const ConvGeom &g, const float *x, const float *f, float *y, cudaS
   return launch_up_v<R, UP, 1>(g, x, f, y, st, 0);
 }
 
+template <int R>
+int launch_square(const ConvGeom &g, const float *x, const float *f, float *y, cudaStream_t st) {
+  int tx, ty;
+  long long blocks;
+  int rc = tile_grid(g, g.OH, g.OW, kTY * 4, kTX * 4, &tx, &ty, &blocks);
+  if (rc) return rc;
+  rc = launch_pdl(direct_square_kernel<R>, dim3((unsigned)blocks), dim3(kThreads), 0, st,
+                  "direct_square_kernel launch", g, x, f, y, tx, ty);
+  if (!rc) count_launches(1);
+  return rc;
+}
+
 int launch_generic(const ConvGeom &g, const float *x, const float *f, float *y,
                    cudaStream_t st) {
   const int tiles_x = (g.OW + kGTW - 1) / kGTW, tiles_y = (g.OH + kGTH - 1) / kGTH;
@@ -666,6 +783,14 @@ int launch_direct(const ConvGeom &g, const float *x, const float *f, float *y,
       default: break;
     }
 #undef CCT_UP_CASE
+  }
+  if (g.up != 1 && g.down == 1 && g.R == g.S) {
+#define CCT_SQUARE_CASE(RR) case RR: return launch_square<RR>(g, x, f, y, st);
+    switch (g.R) {
+      CCT_SQUARE_CASE(1) CCT_SQUARE_CASE(3) CCT_SQUARE_CASE(5) CCT_SQUARE_CASE(7)
+      default: break;
+    }
+#undef CCT_SQUARE_CASE
   }
   return launch_generic(g, x, f, y, st);
 }
