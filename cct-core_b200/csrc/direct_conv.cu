@@ -62,7 +62,8 @@ __global__ void __launch_bounds__(kSmThreads, R == 7 ? 3 : 4)
   const int out_r0 = ty_i * TH, out_c0 = tx_i * TW;
   const int org_r = out_r0 * DOWN - g.low_r;
   const int rows = min(TH, g.OH - out_r0);  // output rows of this tile
-  const TileStage<IN_COLS, PITCH, kSmThreads, VEC> stage(g, out_c0 * DOWN - g.low_c - OFF);
+  const TileStage<IN_COLS, PITCH, kSmThreads, VEC> stage(g, out_c0 * DOWN - g.low_c - OFF,
+                                                         OFF + (min(TW, g.OW - out_c0) - 1) * DOWN + S);
 
   float acc[V][U];
   for (int t = 0; t < g.terms; ++t) {
@@ -160,7 +161,8 @@ __global__ void __launch_bounds__(kSmThreads, R == 7 ? 3 : 4)
 // shared memory before: 1.6 TFLOP/s on 480x640 with sixteen 11x11 filters).
 // Bound: FP32 issue, R*S multiply-adds and R adds per output.
 // A warp's 8-lane float4 phases cover 4 column groups x 2 rows of threads; V
-// odd and a pitch of 4 (mod 8) floats put them on different banks.
+// odd and a pitch of 4 (mod 8) floats put them on different banks.  Seven CTAs an
+// SM up to 9 columns (732x64 by sixty-four 9x9 filters 16.6 us, 18.3 with six).
 constexpr int kWdThreads = 128, kWdU = 8, kWdTX = 8, kWdTY = 16;
 constexpr int kWdTW = kWdTX * kWdU;
 
@@ -174,7 +176,7 @@ inline size_t wide_smem(int R, int S, int V) {
 }
 
 template <int S, int V>
-__global__ void __launch_bounds__(kWdThreads, V > 1 ? 6 : 8)
+__global__ void __launch_bounds__(kWdThreads, V == 1 ? 8 : S > 9 ? 6 : 7)
     direct_wide_kernel(ConvGeom g, const float *__restrict__ x, const float *__restrict__ f,
                        float *__restrict__ y, int tiles_x, int tiles_y) {
   constexpr int U = kWdU, TW = kWdTW, TH = kWdTY * V, PITCH = wide_pitch(S), SP = (S + 3) & ~3;
@@ -198,7 +200,8 @@ __global__ void __launch_bounds__(kWdThreads, V > 1 ? 6 : 8)
   int ip, fp;
   plane_pair(g, o, 0, &ip, &fp);
   {
-    const TileStage<TW + S - 1, PITCH, kWdThreads, false> stage(g, out_c0 - g.low_c);
+    const TileStage<TW + S - 1, PITCH, kWdThreads, false> stage(g, out_c0 - g.low_c,
+                                                                   min(TW, g.OW - out_c0) + S - 1);
     stage.copy(tile, x + (size_t)ip * g.H * g.W, g, out_r0 - g.low_r, rows + R - 1);
     cp_async_commit();
   }
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(kSmThreads, R == 9 ? 2 : R == 7 || UP == 3 ? 3
   const int tx = threadIdx.x % kSmTX, ty = threadIdx.x / kSmTX;
   const int r0 = ty_i * T::TH, c0 = tx_i * T::TW;
   const int rows = min(T::TH, g.H - r0), cols = min(T::TW, g.W - c0);
-  const TileStage<T::IN_COLS, T::PITCH, kSmThreads, false> stage(g, c0 + T::DMIN);
+  const TileStage<T::IN_COLS, T::PITCH, kSmThreads, false> stage(g, c0 + T::DMIN, cols + T::D);
 
   float acc[V][UP][UP][U];
   for (int t = 0; t < g.terms; ++t) {

@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(kTlThreads, V == 8 ? 5 : 8)
   g.W = cols;
   g.border = border;
   {
-    const TileStage<kTlW + RL - 1, PITCH, kTlThreads, false> stage(g, c0 - (RL - 1) / 2);
+    const TileStage<kTlW + RL - 1, PITCH, kTlThreads, false> stage(g, c0 - (RL - 1) / 2,
+                                                                       min(kTlW, cols - c0) + RL - 1);
     stage.copy(img, x + (size_t)pl * rows * cols, g, r0 - (clen - 1) / 2, need);
     cp_async_commit();
   }

@@ -14,7 +14,9 @@ __device__ __forceinline__ int stencil_index(int border, int v, int n) {
 }
 
 // Copies rows x COLS border-mapped values whose corner is (org_r, org_c) into
-// tile[row * PITCH + col].  A thread owns fixed columns of every row it copies,
+// tile[row * PITCH + col]; of a row, only the first `need` columns are read from the
+// field (102 x 8 outputs of a clamped 3x3 DownsampleOutput(2), 361 planes: 44 us
+// reading whole rows, 13 so).  A thread owns fixed columns of every row it copies,
 // so a column is mapped by the border once per tile and an element costs an
 // add and a copy.  (Mapping every element, the way load_tile does, took most
 // of the ~195 instructions per output of a 7x7 clamped stencil.)
@@ -31,13 +33,13 @@ template <int COLS, int PITCH, int THREADS>
 struct TileStage<COLS, PITCH, THREADS, false> {
   static constexpr int KC = (COLS + 31) / 32, STEP = THREADS / 32;
   int sc[KC];    // source column of this lane's k-th column (0 where it reads zero)
-  bool in[KC];
+  bool in[KC];   // the column is needed, and not outside a border that reads zero
 
-  __device__ __forceinline__ TileStage(const ConvGeom &g, int org_c) {
+  __device__ __forceinline__ TileStage(const ConvGeom &g, int org_c, int need) {
 #pragma unroll
     for (int k = 0; k < KC; ++k) {
-      const int c = stencil_index(g.border, org_c + (int)(threadIdx.x & 31) + 32 * k, g.W);
-      in[k] = c >= 0;
+      const int col = (int)(threadIdx.x & 31) + 32 * k, c = stencil_index(g.border, org_c + col, g.W);
+      in[k] = c >= 0 && col < need;
       sc[k] = c < 0 ? 0 : c;
     }
   }
@@ -73,7 +75,7 @@ struct TileStage<COLS, PITCH, THREADS, true> {
   int sc, r0, c0;
   bool in, splat;
 
-  __device__ __forceinline__ TileStage(const ConvGeom &g, int org_c) {
+  __device__ __forceinline__ TileStage(const ConvGeom &g, int org_c, int need) {
     r0 = threadIdx.x / CH;
     c0 = 4 * (threadIdx.x - r0 * CH);
     const int c = org_c + c0, m = stencil_index(g.border, c, g.W);
@@ -82,7 +84,7 @@ struct TileStage<COLS, PITCH, THREADS, true> {
     splat = g.border == CCT_BORDER_CLAMP && m != c;
     in = m >= 0;
     sc = m < 0 ? 0 : m;
-    if (r0 >= STEP) r0 = 1 << 30;  // idle
+    if (r0 >= STEP || c0 >= need) r0 = 1 << 30;  // idle
   }
   __device__ __forceinline__ void chunk(float *d, const float *s, bool ok) const {
     if (splat) {
