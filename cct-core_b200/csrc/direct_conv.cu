@@ -711,6 +711,11 @@ int launch_square(const ConvGeom &g, const float *x, const float *f, float *y, c
   long long blocks;
   int rc = tile_grid(g, g.OH, g.OW, kTY * 4, kTX * 4, &tx, &ty, &blocks);
   if (rc) return rc;
+  // Small grids are better off in the general kernel's quarter tiles, longer the
+  // smaller the filter (up-sampled by 4, us here / there: 1x1 at 400 tiles 13.2 / 12.0,
+  // 800 22.9 / 20.8, 1000 24.3 / 25.1; 3x3 at 296 17.6 / 16.0, 400 18.9 / 19.4; 5x5 at 180
+  // 18.4 / 16.1, 296 18.7 / 23.5; 7x7 at 80 17.9 / 17.1, 120 18.1 / 20.6).
+  if (blocks < (R == 1 ? 900 : R == 3 ? 360 : R == 5 ? 220 : 100)) return 1;
   rc = launch_pdl(direct_square_kernel<R>, dim3((unsigned)blocks), dim3(kThreads), 0, st,
                   "direct_square_kernel launch", g, x, f, y, tx, ty);
   if (!rc) count_launches(1);
@@ -788,11 +793,13 @@ int launch_direct(const ConvGeom &g, const float *x, const float *f, float *y,
 #undef CCT_UP_CASE
   }
   if (g.up != 1 && g.down == 1 && g.R == g.S) {
-#define CCT_SQUARE_CASE(RR) case RR: return launch_square<RR>(g, x, f, y, st);
+    int rc = 1;
+#define CCT_SQUARE_CASE(RR) case RR: rc = launch_square<RR>(g, x, f, y, st); break;
     switch (g.R) {
       CCT_SQUARE_CASE(1) CCT_SQUARE_CASE(3) CCT_SQUARE_CASE(5) CCT_SQUARE_CASE(7)
       default: break;
     }
+    if (rc != 1) return rc;
 #undef CCT_SQUARE_CASE
   }
   return launch_generic(g, x, f, y, st);

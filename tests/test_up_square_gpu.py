@@ -1,5 +1,6 @@
 """Squares over zero-inserted grids: steps and borders past the phase form's, one and
-several terms, at the edges of the 64 x 64 tiles, bit for bit against the FP32 oracle."""
+several terms, at the edges of the 64 x 64 tiles and on both sides of the grid size from
+which they are taken, bit for bit against the FP32 oracle."""
 import numpy as np
 import pytest
 import torch
@@ -27,7 +28,8 @@ def _run(od, x, f, flags=0):
 
 @pytest.mark.parametrize("border,step", [(O.ZERO, 4), (O.CYCLIC, 5), (O.FULL, 2), (O.FULL, 3), (O.VALID, 2), (O.VALID, 4)])
 @pytest.mark.parametrize("R", [1, 3, 5, 7])
-@pytest.mark.parametrize("planes,fplanes,rows,cols", [(0, 0, 33, 65), (3, 0, 8, 7), (0, 5, 16, 16), (2, 2, 21, 40)])
+@pytest.mark.parametrize("planes,fplanes,rows,cols", [(0, 0, 33, 65), (3, 0, 8, 7), (0, 5, 16, 16), (2, 2, 21, 40),
+                                                      (910, 0, 9, 10), (105, 105, 17, 16)])
 def test_planes(planes, fplanes, rows, cols, R, border, step):
     rng = np.random.default_rng(rows + R)
     x = rng.uniform(-1, 1, (max(planes, 1), rows, cols)).astype(np.float32)
