@@ -504,8 +504,15 @@ int launch_separable(int rows, int cols, int planes, const float *x, const float
     // Fewer than 96 TMA tiles leave most SMs idle; the smaller tiles below do not
     // (us: one plane of 512x512, 5 + 5, 32 tiles 3.4 / 2.7; 768x768, 72 tiles 3.5 /
     // 3.3; 1024x1024, 128 tiles 3.7 / 4.4).
+    // Fields that fill less than half of a TMA tile but fit one 64 x 64 tile's columns
+    // and rows are staged as far as they reach there, which pays for flat ones and
+    // for the most taps (us, TMA / small: 3000 of 8x20, 3 + 3 17.3 / 11.8; 1000 of 32x32, 3 +
+    // 3 8.8 / 8.7, 9 + 9 15.6 / 10.9; 1024 of 60x64, 9 + 9 16.3 / 14.3, but 3 + 3 9.6 / 12.3, 5 + 5
+    // 11.0 / 12.4).
     const long long pad = std::min(SepShape<true>::padded(rows, cols), SepShape<false>::padded(rows, cols));
-    if (border == CCT_BORDER_ZERO && (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+    const long long small = (long long)((rows + 63) / 64 * 64) * ((cols + 63) / 64 * 64);
+    const bool wasted = 2 * small <= pad && (rows <= 32 || rlen + clen >= 18);
+    if (border == CCT_BORDER_ZERO && !wasted && (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(y) & 15) == 0 && pad / (64 * 128) * planes >= 96) {
       const int rc = launch_tma_small(rows, cols, planes, x, rf, rlen, cf, clen, orient, y, st);
       if (rc >= 0) return rc;
