@@ -22,6 +22,7 @@ SAMPLE_NONE, SAMPLE_DOWN, SAMPLE_UP = 0, 1, 2
 PREC_FP32, PREC_BF16X3, PREC_BF16X6 = 0, 1, 2
 ALGO_AUTO, ALGO_DIRECT, ALGO_FFT = 0, 1, 2
 FLAG_RELU = 0x1
+BANK_PLAIN, BANK_PAIR, BANK_WIDE, BANK_WIDE_PAIR = range(4)  # forms of Plan.bank
 PLAN_DIRECT, PLAN_FRAME_F32, PLAN_FRAME_BF16X3, PLAN_FFT, PLAN_FILTER_ADJOINT, PLAN_FILTER_ADJOINT_BF16X3 = range(6)
 
 
@@ -93,6 +94,7 @@ SIGNATURES = {
     "cct_conv_plan_create": (_I, [ctypes.POINTER(ConvDesc), ctypes.POINTER(_P)]),
     "cct_conv_plan_destroy": (_I, [_P]),
     "cct_conv_plan_algo": (_I, [_P, _PI32]),
+    "cct_conv_plan_bank": (_I, [_P, _PI32, _PI32, _PI32]),
     "cct_conv_plan_set_static_filter": (_I, [_P, _P]),
     "cct_conv_run": (_I, [_P, _P, _P, _P, _P]),
     "cct_conv_run_host": (_I, [_P, _P, _P, _P, _P]),
@@ -229,6 +231,12 @@ class Plan:
         a = ctypes.c_int32()
         check(LIB.cct_conv_plan_algo(h, ctypes.byref(a)))
         self.algo = a.value
+
+    def bank(self):
+        """(form, halo blocks, tile positions) of a tensor-core filter-bank plan; form -1: it is none."""
+        v = [ctypes.c_int32() for _ in range(3)]
+        check(LIB.cct_conv_plan_bank(self.handle, *(ctypes.byref(x) for x in v)))
+        return tuple(x.value for x in v)
 
     def save(self):
         """Checkpoint record (numpy uint32 words): descriptor + constant filter."""

@@ -11,6 +11,13 @@ constexpr int kBankMaxTaps = 128;   // R * S per tile plan
 constexpr int kBankMaxPhases = 4;   // input phases (DownsampleOutput(2): 2 x 2)
 constexpr int kBankMaxUp = 4;       // UpsampleInput steps the kernel takes
 
+// Forms of a filter block (BankParams::form; cct_conv_plan_bank).
+//   kPlain     64 filters; big and small sums in separate rows
+//   kPair      32 filters x two taps, rows as above (two terms)
+//   kWide      128 filters; big and small sums in separate columns
+//   kWidePair  64 filters x two taps, sums as kWide (three terms)
+enum { kPlain = 0, kPair = 1, kWide = 2, kWidePair = 3 };
+
 struct BankParams {
   ConvGeom g;
   int terms;        // bf16 terms per split value: 2 (BF16X3) or 3 (BF16X6)

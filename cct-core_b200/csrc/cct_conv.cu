@@ -525,6 +525,15 @@ int cct_conv_plan_algo(const cct_conv_plan *p, int32_t *algo) {
   return CCT_OK;
 }
 
+int cct_conv_plan_bank(const cct_conv_plan *p, int32_t *form, int32_t *halo_blocks, int32_t *tile) {
+  if (!p || !form || !halo_blocks || !tile) return set_error(CCT_EINVAL, "null argument");
+  const bool bank = p->algo == ALGO_FRAME_BF16X3 && p->tc.bank;
+  *form = bank ? p->tc.bp.form : -1;
+  *halo_blocks = bank ? p->tc.bp.hblocks : 0;
+  *tile = bank ? p->tc.bp.N : 0;
+  return CCT_OK;
+}
+
 int cct_conv_plan_set_static_filter(cct_conv_plan *p, const float *host_filter) {
   if (!p || !host_filter) return set_error(CCT_EINVAL, "null argument");
   const size_t bytes = p->f_elems * sizeof(float);

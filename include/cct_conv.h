@@ -134,6 +134,12 @@ int cct_conv_plan_algo(const cct_conv_plan *plan, int32_t *algo_out);
  * (generator/DynamicConvolutionGenerator.scala:342-350, 376-405).  After this
  * call cct_conv_run accepts filter == NULL.  host_filter holds
  * filter_planes x filter_rows x filter_cols floats. */
+/* The tensor-core filter-bank kernel's plan: how a block of filters fills its
+ * matrix instructions (0 64 filters, 1 32 filters x two taps, 2 128 filters, 3 64
+ * filters x two taps in three terms; -1: the plan does not run that kernel),
+ * the halo blocks per block of input planes (more than 1: one input phase of
+ * DownsampleOutput each) and the grid positions of a tile. */
+int cct_conv_plan_bank(const cct_conv_plan *plan, int32_t *form, int32_t *halo_blocks, int32_t *tile);
 int cct_conv_plan_set_static_filter(cct_conv_plan *plan, const float *host_filter);
 
 /* One step of the op: device pointers in the planar layout above, enqueued on

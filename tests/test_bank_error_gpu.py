@@ -14,14 +14,14 @@ from cctconv import _lib
 pytestmark = pytest.mark.gpu
 
 
-def _rms_error(B, N, K, size, R, checked=4):
+def _rms_error(B, N, K, size, R, form, checked=4):
     gen = torch.Generator(device="cuda").manual_seed(N + R)
     x = torch.randn((B * N, size, size), device="cuda", generator=gen)
     f = torch.randn((K * N, R, R), device="cuda", generator=gen) * (2.0 / (N * R * R)) ** 0.5
     plan = _lib.Plan(_lib.new_desc(image_rows=size, image_cols=size, image_planes=B * N, filter_rows=R, filter_cols=R,
                                    filter_planes=K * N, batch_size=B, orientation=_lib.CROSS_CORRELATION,
                                    vector_mode=_lib.PROJECT_FRAME_BLOCK_REDUCE_SUM, precision=_lib.PREC_BF16X6))
-    assert plan.algo == _lib.PLAN_FRAME_BF16X3
+    assert plan.bank()[0] == form
     y = torch.full((B * K, size, size), float("nan"), device="cuda")
     plan.run(x.data_ptr(), f.data_ptr(), y.data_ptr(), torch.cuda.current_stream().cuda_stream)
     y = y[:checked].cpu().numpy()
@@ -34,7 +34,8 @@ def _rms_error(B, N, K, size, R, checked=4):
 
 # 128 filters a block; 64 filters x two taps; the plain form; segments that the stages
 # do not divide (144 k-steps)
-@pytest.mark.parametrize("B,N,K,size,R", [(8, 8192, 512, 14, 3), (8, 8192, 64, 28, 5), (1, 2048, 40, 28, 1),
-                                          (8, 256, 192, 52, 3)])
-def test_long_reductions(B, N, K, size, R):
-    assert _rms_error(B, N, K, size, R) <= 1.05 * _rms_error(8, 1024, 64, 28, 1)
+@pytest.mark.parametrize("B,N,K,size,R,form", [
+    (8, 8192, 512, 14, 3, _lib.BANK_WIDE), (8, 8192, 64, 28, 5, _lib.BANK_WIDE_PAIR),
+    (1, 2048, 40, 28, 1, _lib.BANK_PLAIN), (8, 256, 192, 52, 3, _lib.BANK_PLAIN)])
+def test_long_reductions(B, N, K, size, R, form):
+    assert _rms_error(B, N, K, size, R, form) <= 1.05 * _rms_error(8, 1024, 64, 28, 1, _lib.BANK_PLAIN)
