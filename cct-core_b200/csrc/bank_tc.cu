@@ -1064,6 +1064,12 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
   // larger plane block wins (fewer halo hand-offs).
   // dynamic shared memory: 227 KB per CTA less the static barriers and exchange buffers
   const size_t budget = 225 * 1024;
+  // epilogue cycles a position: 64 filters (3 -> 64 planes on 8x 224x224); more where it adds
+  // shifted taps, or stores 128 filters from columns of big and small sums (1.2 to 1.7
+  // times per position over eight layers of 1 to 18 planes, us in 128s / in 64s: 9 -> 145
+  // planes, 5x5 up 4 on 2x 104x36, three terms 113 / 98; 17 -> 106, 1x3 up 2 on 16x 22x123
+  // 65 / 87; 8 -> 87, 3x3 on 16x 109x23, two terms 23 / 28)
+  const double epilogue = p.pair ? 80.0 : form == kWide ? 72.0 : 50.0;
   const int cmax = ((g.n + 15) / 16) * 16;
   bool found = false;
   double best_cost = 0.0, best_waves = 0.0;
@@ -1110,9 +1116,12 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
         const double waves = (double)((items + sms - 1) / sms);
         // a stage of less than ~500 cycles of MMAs takes that long all the same (two
         // terms, 3x3 64 -> 64 on 8x 224x224 down 2: 80 us with 256-cycle stages of N =
-        // 256, 69 with longer ones of a smaller N)
-        const double cost =
-            waves * (std::max(0.5 * N, 32.0 + 0.25 * N) + 8.0) * std::max(1.0, 500.0 / (T * tap_cycles));
+        // 256, 69 with longer ones of a smaller N), unless the tile has so few that its
+        // epilogue takes longer (1x1, 7 -> 9 planes on 20x9: 9.2 us on one tile of 192, 7.2
+        // on three of 64)
+        double floor = std::max(1.0, 500.0 / (T * tap_cycles));
+        if ((double)NU * ((g.n + CB - 1) / CB) * tap_cycles * floor <= epilogue * N) floor = 1.0;
+        const double cost = waves * (std::max(0.5 * N, 32.0 + 0.25 * N) + 8.0) * floor;
         if (!found || cost < best_cost * 0.999 || (cost <= best_cost * 1.001 && CB > best_cb)) {
           p.nbands = nbands;
           p.BW = BW;
@@ -1205,13 +1214,12 @@ bool plan_form(const ConvGeom &g, int terms, int form, bool split, int sms, Bank
   }
   p.pack_bytes = chunks * p.chunk_bytes;
   *out = p;
-  // A tile takes its MMAs or its epilogue, whichever is longer: the epilogue about
-  // 50 cycles a position (3 -> 64 planes on 8x 224x224), 80 where it adds shifted taps.
+  // A tile takes its MMAs or its epilogue, whichever is longer.
   double units = 0.0;
   for (int ph = 0; ph < p.nph_out; ++ph)
     units += u > 1 ? units_of(p.up_rq[ph / u], p.up_sq[ph % u]) : NU;
   const double mmas = best_cost / best_waves * p.NCB * p.KS * p.nmma * units / p.nph_out;
-  *cost_out = best_waves * std::max(mmas, (p.pair ? 80.0 : 50.0) * p.N);
+  *cost_out = best_waves * std::max(mmas, epilogue * p.N);
   return true;
 }
 
