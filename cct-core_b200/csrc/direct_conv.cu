@@ -715,6 +715,12 @@ int launch_square(const ConvGeom &g, const float *x, const float *f, float *y, c
   // smaller the filter (up-sampled by 4, us here / there: 1x1 at 400 tiles 13.2 / 12.0,
   // 800 22.9 / 20.8, 1000 24.3 / 25.1; 3x3 at 296 17.6 / 16.0, 400 18.9 / 19.4; 5x5 at 180
   // 18.4 / 16.1, 296 18.7 / 23.5; 7x7 at 80 17.9 / 17.1, 120 18.1 / 20.6).
+  // So are grids that waste the lower part of their squares, where quarters do not (1x1
+  // up 3, fields of 6x56, 64 rows against 32: 917 / 561 us; 3x3 up 2 BorderFull, 8x9, the
+  // same 44 / 35; but 111x11, 256 against 224: 140 / 185, and 7x7 up 3 BorderFull, 5x91, 64
+  // against 32: 529 / 771).
+  const int tall = (g.OH + 63) / 64 * 64, flat = (g.OH + 15) / 16 * 16;
+  if (tall * 10LL > flat * (R == 1 ? 15LL : R == 3 ? 16 : R == 5 ? 19 : 22)) return 1;
   if (blocks < (R == 1 ? 900 : R == 3 ? 360 : R == 5 ? 220 : 100)) return 1;
   rc = launch_pdl(direct_square_kernel<R>, dim3((unsigned)blocks), dim3(kThreads), 0, st,
                   "direct_square_kernel launch", g, x, f, y, tx, ty);
