@@ -22,7 +22,7 @@
 //
 // The grid is (row tile, column block, reduction split): each CTA reduces a
 // contiguous range of chunks into its accumulator and stores its partial
-// sums; fa_tc_reduce adds the splits in split order, so the result does not
+// sums; fa_tc_reduce adds the splits in a fixed order, so the result does not
 // depend on scheduling.  Within a CTA all 8 warps build every chunk (the
 // next chunks' loads in flight while the current one is converted) into one
 // of kStages stages and arrive on the stage's `full` barrier; one thread
@@ -232,24 +232,26 @@ __global__ void __launch_bounds__(kFaThreads, 2) fa_tc_kernel(const __grid_const
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
-// out[l*C + c](r, s) = sum over splits, in split order, of the partial sums.
-// Adds the splits' partial sums.  A CTA takes 32 adjacent outputs and GROUPS threads
-// share each output's splits (thread k adds splits k, k + GROUPS, .. in order, the
-// sums are then added in order), so the sum's order is fixed and no thread waits
-// for hundreds of loads in turn: one thread per output took 19 us for the 98
-// splits of a 3x3 32 -> 64 weight gradient, as long as a third of the product.
-// 16 threads for many splits, 4 for few (the 29 splits of a 7x7 24 -> 48 one).
+// out[l*C + c](r, s) = the sum of the splits' partial sums.  A CTA takes OUTS adjacent
+// outputs and GROUPS threads share each output's splits (thread k adds splits k, k +
+// GROUPS, .. in order, the sums are then added in order), so the sum's order is fixed
+// and no thread waits for hundreds of loads in turn: one thread per output took 19 us
+// for the 98 splits of a 3x3 32 -> 64 weight gradient, as long as a third of the
+// product.  16 threads for many splits, 4 for few (the 29 splits of a 7x7 24 -> 48 one),
+// one for fewer than 16 or where the outputs alone fill the SMs (whole gradients, us with
+// 4 / 1: 30x30 results of 36 x 23 1x1 gradients, one split, 17.5 / 10.5; 24x24 64 -> 64 with
+// 5x8 results, 14 splits of 164 thousand outputs, 16.7 / 15.0).
 constexpr int kRedOut = 32;
 
-template <int GROUPS>
-__global__ void __launch_bounds__(kRedOut * GROUPS) fa_tc_reduce(const __grid_constant__ FaTcParams p,
-                                                                    float *__restrict__ y) {
-  __shared__ float sums[GROUPS][kRedOut];
+template <int OUTS, int GROUPS>
+__global__ void __launch_bounds__(OUTS * GROUPS) fa_tc_reduce(const __grid_constant__ FaTcParams p,
+                                                              float *__restrict__ y) {
+  __shared__ float sums[GROUPS][OUTS];
   grid_dependency_wait();
   const long long total = (long long)p.L * p.M;
-  const int q = threadIdx.x % kRedOut, k = threadIdx.x / kRedOut;
+  const int q = threadIdx.x % OUTS, k = threadIdx.x / OUTS;
   const size_t step = (size_t)p.Lpad * p.Mpad;
-  for (long long o0 = (long long)blockIdx.x * kRedOut; o0 < total; o0 += (long long)gridDim.x * kRedOut) {
+  for (long long o0 = (long long)blockIdx.x * OUTS; o0 < total; o0 += (long long)gridDim.x * OUTS) {
     const long long o = o0 + q;
     float sum = 0.0f;
     if (o < total) {
@@ -258,14 +260,16 @@ __global__ void __launch_bounds__(kRedOut * GROUPS) fa_tc_reduce(const __grid_co
 #pragma unroll 4
       for (int sp = k; sp < p.splits; sp += GROUPS) sum += src[sp * step];
     }
-    sums[k][q] = sum;
-    __syncthreads();
+    if (GROUPS > 1) {
+      sums[k][q] = sum;
+      __syncthreads();
+    }
     if (k == 0 && o < total) {
 #pragma unroll
       for (int i = 1; i < GROUPS; ++i) sum += sums[i][q];
       y[o] = sum;  // plane l*C + c, pixel (r, s): o = l*M + (c*OH + r)*OW + s
     }
-    __syncthreads();
+    if (GROUPS > 1) __syncthreads();
   }
 }
 
@@ -889,9 +893,13 @@ int launch_fa_tc(const ConvGeom &g, const float *x, const float *f, float *y, fl
   rc = launch_pdl(fa_tc_kernel, dim3((unsigned)grid), dim3(kFaThreads), smem, st, "fa_tc_kernel launch", p);
   if (rc) return rc;
   const long long total = (long long)p.L * p.M;
-  const int blocks = (int)std::min<long long>((total + kRedOut - 1) / kRedOut, 148LL * 64);
-  rc = p.splits >= 64 ? launch_pdl(fa_tc_reduce<16>, dim3(blocks), dim3(kRedOut * 16), 0, st, "fa_tc_reduce launch", p, y)
-                      : launch_pdl(fa_tc_reduce<4>, dim3(blocks), dim3(kRedOut * 4), 0, st, "fa_tc_reduce launch", p, y);
+  auto reduce = [&](auto kern, int outs, int groups) {
+    const int blocks = (int)std::min<long long>((total + outs - 1) / outs, 148LL * 2048 / outs);
+    return launch_pdl(kern, dim3(blocks), dim3(outs * groups), 0, st, "fa_tc_reduce launch", p, y);
+  };
+  rc = p.splits < 16 || total >= 128 * 1024 ? reduce(fa_tc_reduce<256, 1>, 256, 1)
+       : p.splits >= 64                    ? reduce(fa_tc_reduce<kRedOut, 16>, kRedOut, 16)
+                                           : reduce(fa_tc_reduce<kRedOut, 4>, kRedOut, 4);
   if (rc) return rc;
   count_launches(2);
   return CCT_OK;
