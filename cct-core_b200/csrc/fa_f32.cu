@@ -14,8 +14,8 @@
 // bit-identical to the FP32 oracle.
 //
 // fa_quad_kernel: the main path, described below.
-// fa_rows_kernel (fields too wide for its shared memory): a CTA serves one
-// image b, kCG input planes and kLG gradient planes.  It streams the gradient
+// fa_rows_kernel (fields too wide for its shared memory, gradients of few rows):
+// a CTA serves one image b, kCG input planes and kLG gradient planes.  It streams the gradient
 // rows i = 0.. through
 // shared memory together with a ring of the OH image rows each step needs
 // (cp.async, the next rows landing while the current ones are used), so
@@ -449,7 +449,16 @@ int launch_fa_f32(const ConvGeom &g, const float *x, const float *f, float *y, f
   // 5x5 32 -> 64 on 16x 64x64 248 / 224)
   const int nw = qblocks > 400 ? 4 : quad_smem(g, 16) <= kQuadSmemMax ? 16 : quad_smem(g, 8) <= kQuadSmemMax ? 8 : 4;
   const size_t qsmem = quad_smem(g, nw);
-  if (g.OH <= kFaMaxS && qsmem <= kQuadSmemMax && qblocks <= 0x7fffffffLL && (long long)g.n * g.OH < (1 << 30)) {
+  // Gradients of one to three rows leave most of a step's warps idle and its sums'
+  // exchange in the open: fa_rows_kernel is the faster one for narrow results, once the
+  // grid is more than a wave of latency (us, quad / rows: 1x1 on 16x 38 -> 64 with 5x5
+  // results 13.2 / 11.0, 1x4 on 8x 38 -> 26 with 3x3 6.7 / 4.8, 1x8 on 64 -> 64 with 1x1 5.9 / 4.3,
+  // 2x2 on 8x 38 -> 26 with 5x5 9.2 / 7.6; but 8x8 results 5.9 / 10.8, 2x2 on 8 -> 8 with 5x5
+  // 4.1 / 6.5).
+  const bool flat = g.OW <= 5 && g.R <= (g.OW <= 3 ? 3 : 2) && (qblocks >= 150 || (g.R == 1 && g.OW <= 3)) &&
+                    rsmem <= kRowsSmemMax;
+  if (!flat && g.OH <= kFaMaxS && qsmem <= kQuadSmemMax && qblocks <= 0x7fffffffLL &&
+      (long long)g.n * g.OH < (1 << 30)) {
 #define CCT_FA_QUAD_CASE(SS)                                                                                  \
   case SS: {                                                                                                  \
     const auto kern = nw == 16 ? fa_quad_kernel<SS, 16> : nw == 8 ? fa_quad_kernel<SS, 8> : fa_quad_kernel<SS, 4>; \
