@@ -3,10 +3,14 @@
 // (ConvolveHyperKernel.scala:153-199, 319-340, 574-645), every border policy
 // (:235-317), DownsampleOutput(1, 2) (:205-223), UpsampleInput(2-4)
 // (:206-212, 405-459, as one sub-filter per output phase), any field width.
-// Banks of at most 32 filters put two taps of a filter row into each MMA
-// (paired taps: tap b's sums are read one grid position to the right).
+// A block of filters fills the MMAs in one of four forms (bank_tc.h).  The plain one
+// takes 64 filters, with the layout and the zero rows described here.  Banks of at
+// most 32 filters put two taps of a filter row into each MMA (paired taps: tap b's
+// sums are read one grid position to the right).  The wide forms, 128 filters or 64
+// filters x two taps, keep big and small sums in separate accumulator columns and have
+// no zero rows (below block_term).
 //
-// GEMM view, per image b and block of 64 filters:
+// GEMM view, per image b and block of filters:
 //   D[filter k][position p] = sum over (plane c, tap t) F[k][c, t] * X[c][p + off(t)]
 // M = the filter block, N = a tile of output positions, reduction = planes x
 // taps.  Positions live on a padded output grid of pitch P = BW + (S-1)/step
@@ -18,8 +22,8 @@
 // computed and discarded ((S-1)/P of the work).  DownsampleOutput(2) holds
 // the input as its four polyphase components, each a stride-1 grid.
 //
-// Split precision.  x = xh + xl (+ xm) and f likewise, each term bf16.  The
-// filter operand of one MMA is 128 rows: rows 0-63 ("big") multiply into the
+// Split precision.  x = xh + xl (+ xm) and f likewise, each term bf16.  In the plain
+// form the filter operand of one MMA is 128 rows: rows 0-63 ("big") multiply into the
 // hi*hi sum only, rows 64-127 ("small") into the correction products:
 //   2 terms (BF16X3): [Fh; Fl] x Xh  and  [0; Fh] x Xl
 //                     -> big hh, small lh + hl
@@ -33,8 +37,9 @@
 // exactly 0) fill the big half of the other MMAs.  For long reductions the
 // accumulator is also promoted: every seg_stages stages the epilogue adds it
 // into an FP32 running sum (RN, CUDA cores) and the next MMA starts it
-// afresh, which bounds the accumulation error by the segment length.  The
-// epilogue adds each filter's big and small rows.
+// afresh, which bounds the accumulation error by the segment length; the
+// wide forms' small sums every few segments.  The epilogue adds each filter's big and
+// small sums.
 //
 // Warp roles (one persistent CTA per SM, 640 threads):
 //   warps 0-9   converters: for each (tile, plane block) fill a halo buffer:
@@ -441,7 +446,8 @@ template <int TERMS, int FORM, bool CB16>
 __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_constant__ BankParams p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ Bars bars;
-  // epilogue exchange: 4 groups of 2 part tiles, or (paired taps) 2 groups of 4
+  // epilogue exchange: 4 groups of 2 part tiles, (paired taps) 2 groups of 4, or (128
+  // filters) 8 groups of 1
   __shared__ __align__(16) float xch[8 * kXchFloats];
   __shared__ uint32_t unit_boff[kBankMaxTaps];  // MMA warp: B operand offset of each unit
   const ConvGeom &g = p.g;

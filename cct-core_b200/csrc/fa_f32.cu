@@ -5,21 +5,21 @@
 // The block-reduced form sums the B images of each w in order.
 //
 // The result planes are tiny (the filter's size) and the reduction is long
-// (the whole gradient plane).  Each thread owns one (input plane c, gradient
-// plane l, result row r) and keeps the result row's S outputs in registers
-// while it walks the gradient; the image row it needs slides through a
-// register window, so each tap costs one image load and one gradient load for
-// S multiply-adds.  Per output the order is the reference's: an fma chain over
+// (the whole gradient plane).  A thread owns a (input plane c, result row r)
+// and one gradient plane l (fa_rows_kernel, fa_f32_kernel) or four
+// (fa_quad_kernel), and keeps the result rows' S outputs in registers while it
+// walks the gradient; the image row it needs slides through a register window, so
+// an image load feeds S multiply-adds per gradient plane.  Per output the order is the reference's: an fma chain over
 // j from 0 per gradient row, row sums added in order, so the result is
 // bit-identical to the FP32 oracle.
 //
 // fa_quad_kernel: the main path, described below.
 // fa_rows_kernel (fields too wide for its shared memory, gradients of few rows):
-// a CTA serves one image b, kCG input planes and kLG gradient planes.  It streams the gradient
-// rows i = 0.. through
-// shared memory together with a ring of the OH image rows each step needs
-// (cp.async, the next rows landing while the current ones are used), so
-// every image row and gradient row is read from L2 once per CTA.
+// a CTA serves one image b, kCG input planes and kLG gradient planes.  It
+// streams the gradient rows i = 0.. through shared memory together with a ring
+// of the OH image rows each step needs (cp.async, the next rows landing while
+// the current ones are used), so every image row and gradient row is read from
+// L2 once per CTA.
 // fa_f32_kernel: the fallback for image rows too wide to stage; one CTA per
 // (b, l) with the gradient plane in shared memory and image rows read
 // through L1.
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kCG * kLG * kFaMaxS)
 // fa_quad_kernel (the main path): a lane owns one (input plane, result row)
 // and four gradient planes, so an image value feeds 4 S multiply-adds and a
 // float4 of the four planes' gradients comes as one broadcast read; a warp
-// owns a gradient row i of the step, kQRows warps the step's rows.  Row sums
+// owns a gradient row i of the step, NW warps the step's rows.  Row sums
 // meet in shared memory and are added in row order by the thread that keeps
 // the output, so splitting the rows over warps does not change the order.
 // Gradient planes l, l+1 advance together in packed fma.rn.f32x2 (each lane

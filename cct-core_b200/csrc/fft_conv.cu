@@ -51,9 +51,10 @@ __host__ __device__ constexpr int col_width(int Fr) {
   return Fr == 4096 ? 2 : Fr / 16 * 4 >= 64 ? 4 : 64 / (Fr / 16);
 }
 // Column threads to keep resident per SM: 1024 (64 registers a thread, a few
-// spilled) for the long columns that fill the SMs; up to 1024 rows a plane has at
-// most 129 CTAs, so 512 and no spills (512x512: 20.8 us a convolution, 18.7 so;
-// 2048x2048: 56.7, 62.0 so).
+// spilled) for columns of more than 1024 rows, 512 and no spills up to that (31x31 cyclic
+// or clamp, us a convolution with 1024 / 512: 512x512 20.8 / 18.7, 1024x2048 45.9 / 38.0, 480x640
+// 26.6 / 23.7; many CTAs: 16 planes of 1024x1024 152 / 148, 64 of 480x640 275 / 265, 8 of
+// 512x4096 clamp 412 / 417; 2048x2048, 1024 against 512, 56.7 / 62.0).
 __host__ __device__ constexpr int col_residency(int Fr) { return Fr <= 1024 ? 512 : 1024; }
 // Shared-memory stride of a column in complex values: a warp holds 32/CW
 // consecutive elements of each of CW columns, so a stride of 32/CW (mod 16)

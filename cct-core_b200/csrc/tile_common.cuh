@@ -1,5 +1,5 @@
 // Device helpers shared by the direct and frame convolution kernels: border
-// extension and the halo-tile loaders.
+// extension, the synchronous halo-tile load and asynchronous copies.
 #pragma once
 
 #include "cct_internal.h"
@@ -69,8 +69,7 @@ __device__ __forceinline__ void load_tile(float *tile, int pitch, int rows,
   }
 }
 
-// Asynchronous (cp.async) variant of load_tile: 4-byte copies with zero fill
-// (src-size 0) for positions that read zero.  The caller commits and waits.
+// cp.async of 4 bytes, or 4 zero bytes (src-size 0).  The caller commits and waits.
 __device__ __forceinline__ void cp_async_f32(float *dst, const float *src,
                                              bool valid) {
   const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
@@ -90,35 +89,6 @@ __device__ __forceinline__ void cp_async_commit() {
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ void load_tile_async(float *tile, int pitch,
-                                                int rows, int cols,
-                                                const float *__restrict__ src,
-                                                const ConvGeom &g, int org_r,
-                                                int org_c) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nwarps = blockDim.x >> 5;
-  const bool interior = g.up == 1 && org_r >= 0 && org_c >= 0 &&
-                        org_r + rows <= g.H && org_c + cols <= g.W;
-  if (interior) {
-    for (int tr = warp; tr < rows; tr += nwarps) {
-      const float *s = src + (size_t)(org_r + tr) * g.W + org_c;
-      float *d = tile + tr * pitch;
-      for (int tc = lane; tc < cols; tc += 32) cp_async_f32(d + tc, s + tc, true);
-    }
-  } else {
-    for (int tr = warp; tr < rows; tr += nwarps) {
-      const int sr = source_index(g.border, org_r + tr, g.H, g.up);
-      const float *s = src + (size_t)(sr < 0 ? 0 : sr) * g.W;
-      float *d = tile + tr * pitch;
-      for (int tc = lane; tc < cols; tc += 32) {
-        const int sc = source_index(g.border, org_c + tc, g.W, g.up);
-        const bool ok = sr >= 0 && sc >= 0;
-        cp_async_f32(d + tc, ok ? s + sc : src, ok);
-      }
-    }
-  }
 }
 
 }  // namespace cct
