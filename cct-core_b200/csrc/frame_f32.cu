@@ -291,8 +291,12 @@ int launch(const ConvGeom &g, const float *x, const float *f, float *y, cudaStre
   const long long blocks16 = (long long)((g.OW + kTW - 1) / kTW) * ((g.OH + kTH - 1) / kTH) * g.batch *
                              ((g.groups + 15) / 16);
   const bool full16 = (g.groups + 15) / 16 * 16 * 4 <= g.groups * 5;  // at most a fifth of the planes idle
-  if constexpr (R <= 3) {
-    if (blocks16 >= 128 && full16) return launch_k<R, S, DOWN, true, 8, 2>(g, x, f, y, st);
+  // DownsampleOutput(2) stages four times the field per output, so there every size takes 16
+  // planes, 1x1 from 40 CTAs on (us, 16 / 4, clamp: 1x1 10 -> 47 planes on 16x 40x14 14 / 31; 5x5
+  // 23 -> 117 on 16x 48x34 96 / 166; 7x7 8 -> 143 on 8x 40x80 61 / 101; at 192 CTAs and zero
+  // borders about even: 5x5 25 -> 44 on 16x 40x114 82 / 70).
+  if constexpr (R <= 3 || DOWN == 2) {
+    if (blocks16 >= (R == 1 && DOWN == 2 ? 40 : 128) && full16) return launch_k<R, S, DOWN, true, 8, 2>(g, x, f, y, st);
   }
   return launch_k<R, S, DOWN, true, 4, 1>(g, x, f, y, st);
 }
