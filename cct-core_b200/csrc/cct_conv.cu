@@ -68,7 +68,6 @@ unsigned *device_error_word() {
 }
 
 int raise_smem_limit(const void *kernel, size_t bytes, const char *what) {
-  if (bytes <= 48 * 1024) return CCT_OK;
   static std::mutex mu;
   static std::map<std::pair<const void *, int>, size_t> limits;  // by kernel and device
   int dev = 0;

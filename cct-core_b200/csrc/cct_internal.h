@@ -117,7 +117,8 @@ bool frame_f32_supported(const ConvGeom &g);
 int launch_frame_f32(const ConvGeom &g, const float *x, const float *f,
                      float *y, cudaStream_t stream);
 // Raises a kernel's dynamic shared-memory limit on the current device to at least
-// `bytes` (nothing to do up to 48 KB); never lowers it.  The limit belongs to the
+// `bytes`; never lowers it.  Small sizes too: what a kernel may use unasked is 48 KB less
+// its static shared memory.  The limit belongs to the
 // kernel, not to a launch, and its sizes depend on the call: set to each call's own
 // size, a thread about to launch a large one could have it lowered by another
 // thread's small one.
