@@ -669,11 +669,13 @@ __global__ void __launch_bounds__(kThreads, 1) bank_tc_kernel(const __grid_const
             tc_fence_after();
             seg_left = min(p.seg_stages, tstages - done);
             first = true;
-            if (small_left == 0) {
-              small_left = p.small_segs;
-              first_small = true;
+            if (wide_form(FORM)) {
+              if (small_left == 0) {
+                small_left = p.small_segs;
+                first_small = true;
+              }
+              --small_left;
             }
-            --small_left;
           }
           failed = __any_sync(0xffffffffu, !mbar_wait(&bars.full[s], sph, p.err));
           if (failed) break;

@@ -721,7 +721,7 @@ int launch_square(const ConvGeom &g, const float *x, const float *f, float *y, c
   // against 32: 529 / 771).
   const int tall = (g.OH + 63) / 64 * 64, flat = (g.OH + 15) / 16 * 16;
   if (tall * 10LL > flat * (R == 1 ? 15LL : R == 3 ? 16 : R == 5 ? 19 : 22)) return 1;
-  if (blocks < (R == 1 ? 900 : R == 3 ? 360 : R == 5 ? 220 : 100)) return 1;
+  if (blocks < (R == 1 ? 900 : R == 3 ? 360 : R == 5 ? 220 : 88)) return 1;
   rc = launch_pdl(direct_square_kernel<R>, dim3((unsigned)blocks), dim3(kThreads), 0, st,
                   "direct_square_kernel launch", g, x, f, y, tx, ty);
   if (!rc) count_launches(1);
